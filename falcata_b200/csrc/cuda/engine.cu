@@ -218,10 +218,10 @@ CudaEngine::CudaEngine(const Config& cfg, const Dataset* train, const ObjectiveF
   }
   cand_.Alloc(static_cast<size_t>(NL) * std::max<size_t>(1, owned_features_.size())); cand_.Zero(stream_);
   root_child_.Alloc(1); child_done_.Alloc(2 * static_cast<size_t>(NL) + 2); child_done_.Zero(stream_); level_done_.Alloc(1); level_done_.Zero(stream_);
-  split_done_.Alloc(NL + 1); split_done_.Zero(stream_);
   hist_tasks_.Alloc(NL); hist_status_.Alloc(1); hist_status_.Zero(stream_); h_hist_status_.Alloc(1); *h_hist_status_.get() = 0;
   const size_t max_chunks = static_cast<size_t>(n_) / kPartChunk + NL + 1;
   bits_.Alloc(max_chunks * (kPartChunk / 32)); chunk_left_.Alloc(max_chunks); split_left_total_.Alloc(NL);
+  chunk_words_.Alloc(max_chunks); chunk_words_.Zero(stream_);
   const size_t blob = static_cast<size_t>(NL) * (sizeof(PartSplit) + sizeof(ChildInit) + 2 * sizeof(FindChild)) + 256;
   level_blob_.Alloc(blob); h_level_blob_.Alloc(blob);
   features_.Alloc(std::max(1, train->num_features)); sub_features_.Alloc(std::max(1, train->num_features));

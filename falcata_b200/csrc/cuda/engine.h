@@ -124,6 +124,7 @@ class CudaEngine : public DeviceEngine {
   DevBuf<char> level_blob_; PinnedBuf<char> h_level_blob_;
   DevBuf<HistTask> hist_tasks_; DevBuf<unsigned int> hist_status_; PinnedBuf<unsigned int> h_hist_status_;
   DevBuf<unsigned int> bits_; DevBuf<int> chunk_left_, split_left_total_;
+  DevBuf<unsigned long long> chunk_words_; unsigned int part_epoch_ = 0;   // look-back words of the one-launch partition, epoch of its last launch
   DevBuf<int> features_, sub_features_;
   // exact leaf-wise growth (grow_policy=leaf): the device grows up to grow_leaves_ leaves, the host keeps the best num_leaves
   bool leafwise_ = false; int grow_leaves_ = 0;
@@ -156,7 +157,7 @@ class CudaEngine : public DeviceEngine {
   bool fast_score_ok_ = false, score_done_ = false; double cur_shrinkage_ = 1.0; float* cur_score_ = nullptr;
   DevBuf<LevelCtrl> ctrl_; DevBuf<int> frontier_; DevBuf<SplitJournal> journal_;   // ctrl_: two level records (a ring, see TrainTree)
   DevBuf<FindChild> root_child_;                                   // the root's search descriptor
-  DevBuf<unsigned int> child_done_, level_done_, split_done_;     // arrival counters of the fused kernels (zero between launches)
+  DevBuf<unsigned int> child_done_, level_done_;     // arrival counters of the fused kernels (zero between launches)
   PinnedBuf<LevelCtrl> h_ctrl_; PinnedBuf<SplitJournal> h_journal_; PinnedBuf<LeafInfo> h_root_;
   // bagging (device-drawn; -1 = no bag drawn)
   double bag_fraction_ = 1.0; int bag_freq_ = 0, bag_seed_ = 0;

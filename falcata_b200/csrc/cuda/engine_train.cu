@@ -182,6 +182,7 @@ Tree* CudaEngine::TrainTree(int class_id, int tree_index) {
     if (data_parallel()) fabric_->AllReduce(kFabricSumF64, root_sums_d_.get(), root_sums_d_.get(), 2, stream_);
   }
   const bool bagged = bag_active_;
+  const bool one_launch_part = plan_.fused_scan && !feature_parallel_ && use_ctrl_;   // feature-parallel: the bit words travel between the ranks
   {
     // root leaf record, level-record ring, frontier, the root's construct task and search descriptor: one small kernel
     TreeInitArgs ti;
@@ -194,7 +195,7 @@ Tree* CudaEngine::TrainTree(int class_id, int tree_index) {
     LaunchInitTree(ti, stream_);
   }
   if (bagged) FB_CUDA(cudaMemcpyAsync(idx_[0].get(), bag_idx_.get(), sizeof(int) * static_cast<size_t>(root_count_), cudaMemcpyDeviceToDevice, stream_));
-  else LaunchInitIndices(idx_[0].get(), n_, stream_);
+  else if (!one_launch_part) LaunchInitIndices(idx_[0].get(), n_, stream_);   // otherwise the root's partition numbers the rows itself
   clock_.End(stream_);
 
   // ---- common launch descriptors ----
@@ -376,7 +377,7 @@ Tree* CudaEngine::TrainTree(int class_id, int tree_index) {
     pa.splits = ca.splits; pa.num_splits = max_splits; pa.total_chunks = n_ / kPartChunk + max_splits; pa.bits = bits_.get(); pa.chunk_left = chunk_left_.get();
     pa.split_left_total = split_left_total_.get(); pa.leaves = leaves_.get(); pa.child_init = ca.child_init; pa.hist_tasks = hist_tasks_.get(); pa.rows_per_block = rpb;
     pa.world = dp ? world_ : 1;
-    pa.fused_scan = (plan_.fused_scan && !feature_parallel_) ? 1 : 0; pa.split_done = split_done_.get();
+    pa.chunk_words = one_launch_part ? chunk_words_.get() : nullptr;
     if (dp) for (int r = 0; r < world_; ++r) pa.peer_counts[r] = fabric_->Ptr<int>(r, off_counts_) + static_cast<size_t>(rank_) * NL;
     if (feature_parallel_) SetupBitmapBroadcast(&pa);
     ha.identity_root = 0; ha.rows_per_block = rpb; ha.num_tasks = max_splits; ha.total_blocks = n_ / rpb + max_splits;
@@ -392,7 +393,8 @@ Tree* CudaEngine::TrainTree(int class_id, int tree_index) {
       if (num_sets_ > 0) LaunchPathBits(lc, journal_.get(), dd_->feature_meta.get(), path_bits_.get(), path_words_, max_splits, stream_);
       if (feature_parallel_) { pa.bc_sig.epoch = fabric_->NextEpoch(); pa.bc_wait.epoch = pa.bc_sig.epoch; }
       clock_.Begin(st_part_, stream_);
-      LaunchPartitionFlags(pa, stream_); LaunchPartitionScanSetup(pa, stream_); LaunchPartitionScatter(pa, stream_);
+      pa.identity = level == 1 && !bagged ? 1 : 0; pa.epoch = ++part_epoch_;
+      LaunchPartition(pa, stream_);
       clock_.End(stream_);
       construct_and_find();
     };
@@ -518,7 +520,7 @@ Tree* CudaEngine::TrainTree(int class_id, int tree_index) {
     if (dp) for (int r = 0; r < world_; ++r) pa.peer_counts[r] = fabric_->Ptr<int>(r, off_counts_) + static_cast<size_t>(rank_) * NL;
     if (feature_parallel_) { SetupBitmapBroadcast(&pa); pa.bc_sig.epoch = fabric_->NextEpoch(); pa.bc_wait.epoch = pa.bc_sig.epoch; }
     clock_.Begin(st_part_, stream_);
-    LaunchPartitionFlags(pa, stream_); LaunchPartitionScanSetup(pa, stream_); LaunchPartitionScatter(pa, stream_);
+    LaunchPartition(pa, stream_);
     clock_.End(stream_);
     ha.num_tasks = S; ha.total_blocks = std::max(1, block_cursor);
     fa.children = reinterpret_cast<const FindChild*>(db + (sizeof(PartSplit) + sizeof(ChildInit)) * S); fa.num_children = 2 * S;

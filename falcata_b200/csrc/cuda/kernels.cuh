@@ -256,8 +256,9 @@ struct PartArgs {
   int rows_per_block;
   int world; int* peer_counts[kMaxRanks];   // world > 1: address of counts[this rank][0] inside every rank's heap
   const LevelCtrl* ctrl;     // non-null: num_splits / total_chunks come from the device controller
-  int fused_scan;            // 1: the last chunk block of each split runs the scan + set-up step (every split has >= 1 chunk)
-  unsigned int* split_done;  // [splits] chunk blocks finished per split (zero between launches)
+  unsigned long long* chunk_words;   // non-null: one launch per level; [chunks] look-back words, valid when they carry `epoch`
+  unsigned int epoch;                // one-launch form: differs from that of every earlier launch on the same words (never 0)
+  int identity;                      // one-launch form: the windows hold the rows in order (root of an unbagged tree), idx is not read
   // ---- feature-parallel bitmap broadcast (bc_world > 1) ----
   // Every rank holds all rows but only the histograms of the features it owns. The rank that owns a
   // split's feature computes the go-left bit words of the leaf's rows and stores them, with the chunk
@@ -267,6 +268,7 @@ struct PartArgs {
   unsigned int* peer_bits[kMaxRanks]; int* peer_chunk_left[kMaxRanks];
   FabricSignal bc_sig; FabricWait bc_wait;
 };
+void LaunchPartition(const PartArgs& a, cudaStream_t s);   // one launch, or flags + scan + scatter when chunk_words is null
 void LaunchPartitionFlags(const PartArgs& a, cudaStream_t s);
 void LaunchPartitionScanSetup(const PartArgs& a, cudaStream_t s);
 void LaunchPartitionScatter(const PartArgs& a, cudaStream_t s);

@@ -203,7 +203,7 @@ struct Plan {
   bool hist_tc = false;          // root level of the quantized construct on the tensor cores (one-hot tcgen05 instance, 1 GPU)
   bool device_controller = true; // split arbitration on the device (no per-level host decision)
   bool fused_tail = true;        // split search, per-leaf argmax, cross-rank argmax and the level controller in ONE launch
-  bool fused_scan = true;        // the partition's scan + child set-up step inside the flags launch (last chunk block of each split)
+  bool fused_scan = true;        // the row partition of a level in one launch (off: flags, scan + child set-up, scatter)
   bool pack4 = true;             // 4-bit row storage when every group has <= 16 bins
   bool compact_view = true;      // per-tree gather of feature_fraction-sampled columns
   bool gh_in_row = false;        // packed gradient word stored next to the row's bins (measured slower on B200: the separate 4 B/row array stays L2-resident)
