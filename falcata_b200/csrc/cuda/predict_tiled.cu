@@ -1,7 +1,14 @@
 // K7, tiled form: a block stages a tile of rows in shared memory once (feature-major, so that the lane that owns a
 // row always reads its own bank) and walks it through the whole forest; the trees stream through shared memory in
 // chunks of a few trees, double-buffered with asynchronous copies, as 8-byte nodes whose two children sit next to
-// each other. Every thread owns one row and keeps eight tree walks in flight.
+// each other. The block's threads are (row, tree slice) pairs: kWalks walks in flight per thread, and the slices add warps
+// where the shared memory has no room for more rows.
+//
+// What bounds it: instructions per step of a walk. A node holds everything as ready-made offsets into the block's shared
+// memory (feature row, left child) and a leaf is a node that leads to itself - its feature row holds -infinity, which goes
+// left everywhere - so a step is shift, mask, load, mask, compare, add, load, without a test for the end.
+// Measured: 4M rows x 136 features, 500 trees of 255 leaves, 41.0 -> 24.4 ms against 256 threads with eight walks each and
+// nodes of indices; 200k rows x 100 features, 500 trees of 127 leaves with missing values, 3.8 -> 2.1 ms.
 //
 // Parity: python-package/falcata/basic.py:L5112-5163 (device predict route: raw score, converted score, leaf index),
 // include/Falcata/tree.h:L361-439 (numerical decision with missing-value handling). Forests with categorical splits,
@@ -10,6 +17,7 @@
 #include <cuda_pipeline.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <limits>
 #include <vector>
@@ -20,18 +28,22 @@ namespace fb {
 
 namespace {
 
-// value: threshold of an internal node, output of a leaf.
-// meta:  bits 0-15 feature slot (0xFFFF: leaf), bits 16-28 index of the left child inside the tree (the right child
-//        is the next node; for a leaf: the leaf's index), bit 29 default-left, bits 30-31 missing type.
+// value: threshold of an internal node; output of a leaf (leaf-index prediction: the leaf's index, as bits).
+// meta:  bits 16-31 feature slot: the feature's row of the tile, counted in rows from the start of the block's shared memory;
+//        bits 3-15 byte offset of the left child in its chunk (a multiple of 8; the right child is the next node, a leaf
+//        leads to itself); bits 1-2 missing type (kLeafType: a leaf); bit 0 default-left.
 struct PackedNode { float value; unsigned int meta; };
 static_assert(sizeof(PackedNode) == 8, "8-byte nodes");
 
-constexpr int kTileThreads = 256;          // rows of a tile = threads of a block
-constexpr int kChunkBytes = 32 * 1024;     // one buffer of the tree ring
-constexpr unsigned int kLeafSlot = 0xFFFFu;
-constexpr int kWalks = 8;                  // tree walks a thread keeps in flight
+constexpr int kPredictThreads = 512;        // threads of a block = rows of its tile x tree slices
+constexpr int kMaxTileRows = 256;
+constexpr int kTreeBytes = 32 * 1024;       // a tree and its root word must fit this much; also the smaller chunk size
+constexpr int kPredictSmem = 220 * 1024;
+constexpr unsigned int kLeafType = 3;
+constexpr unsigned int kChildMask = 0xFFF8u;
+constexpr int kWalks = 4;                   // tree walks a thread keeps in flight
 
-struct ChunkDesc { long long offset; int bytes; int ntrees; int cls; int first_tree; };   // blob offset (16-byte aligned)
+struct ChunkDesc { long long offset; int bytes; int ntrees; int roots; int cls; int first_tree; int pad; };   // blob offset (16-byte aligned); roots: offset of the trees' root words
 
 template <typename T> __device__ inline float ToF(T v) { return static_cast<float>(v); }
 template <> __device__ inline float ToF<__half>(__half v) { return __half2float(v); }
@@ -41,56 +53,64 @@ template <> __device__ inline float ToF<__half>(__half v) { return __half2float(
 template <bool PLAIN>
 __device__ __forceinline__ bool GoLeft(float v, float thr, unsigned int meta) {
   if (PLAIN) return v <= thr;
-  const unsigned int mt = meta >> 30;
+  const unsigned int mt = (meta >> 1) & 3u;
   const bool nan = isnan(v);
   if (nan && mt != 2u) v = 0.f;
   const bool use_default = (mt == 1u && fabsf(v) <= 1e-35f) || (mt == 2u && nan);
-  return use_default ? ((meta >> 29) & 1u) != 0u : v <= thr;
+  return use_default ? (meta & 1u) != 0u : v <= thr;
 }
 
 // LEAF: write the leaf index of every (row, tree) instead of summing outputs.
+// Shared memory: [2][chunk_bytes] tree ring (chunk_bytes a power of two), [num_used + 1][tile_rows] floats (the last row is the
+// leaves' -infinity), [kPredictThreads] doubles. log_rows: log2(tile_rows), 5..8.
 template <typename T, bool LEAF, bool PLAIN>
-__global__ void __launch_bounds__(kTileThreads, 1)
-PredictTiledKernel(const unsigned char* __restrict__ blob, const ChunkDesc* __restrict__ chunks, int num_chunks, const int* __restrict__ used, int num_used,
-                   const T* __restrict__ data, int nrow, int ncol, int row_major, int num_class, int trees_total, float inv_avg, float* __restrict__ out,
-                   int* __restrict__ out_leaf) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  unsigned char* ring = smem;                                                   // [2][kChunkBytes]
-  float* rows_s = reinterpret_cast<float*>(smem + 2 * kChunkBytes);             // [num_used][kTileThreads]
+__global__ void __launch_bounds__(kPredictThreads, 1)
+PredictTiledKernel(const unsigned char* __restrict__ blob, const ChunkDesc* __restrict__ chunks, int num_chunks, int chunk_bytes, const int* __restrict__ used, int num_used,
+                   const T* __restrict__ data, int nrow, int ncol, int row_major, int log_rows, int num_class, int trees_total, float inv_avg, float* __restrict__ out) {
+  extern __shared__ __align__(1024) unsigned char smem[];
+  const int tile_rows = 1 << log_rows, slices = kPredictThreads >> log_rows;
+  unsigned char* ring = smem;
+  float* rows_s = reinterpret_cast<float*>(smem + 2 * chunk_bytes);
+  double* sums = reinterpret_cast<double*>(smem + 2 * chunk_bytes + (num_used + 1) * tile_rows * 4);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int num_tiles = (nrow + kTileThreads - 1) / kTileThreads;
+  const int r = tid & (tile_rows - 1), slice = tid >> log_rows;
+  // a slot's byte offset is slot * tile_rows * 4: shift it out of the meta word, the row's own offset fills the low bits
+  const unsigned int slot_shift = 16 - (log_rows + 2), slot_mask = ~(static_cast<unsigned int>(tile_rows) * 4u - 1u), row_bytes = r * 4;
+  const int num_tiles = (nrow + tile_rows - 1) >> log_rows;
+  for (int i = tid; i < tile_rows; i += kPredictThreads) rows_s[num_used * tile_rows + i] = __int_as_float(0xff800000);   // -infinity
   for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
-    const int row0 = tile * kTileThreads;
-    const int row = row0 + tid;
+    const int row0 = tile << log_rows;
+    const int row = row0 + r;
     __syncthreads();   // the previous tile's walks are over before its rows and ring buffers are overwritten
     // ---- stage the tile: rows_s[j][r] = value of used feature j in row row0 + r ----
     if (!row_major) {
-      for (int j = 0; j < num_used; ++j) {
+      for (int j = slice; j < num_used; j += slices) {
         float v = row < nrow ? ToF<T>(data[static_cast<size_t>(used[j]) * nrow + row]) : 0.f;
         if (PLAIN && isnan(v)) v = 0.f;
-        rows_s[j * kTileThreads + tid] = v;
+        rows_s[j * tile_rows + r] = v;
       }
     } else {
-      // 32 x 32 pieces: read with the lanes along the features (coalesced), turn in a padded scratch piece that
-      // borrows the still unused ring, write with the lanes along the rows (conflict-free)
-      float* scratch = reinterpret_cast<float*>(ring) + warp * (32 * 33);
+      // 16 rows x 32 features: read with the lanes along the features (coalesced), turn in a padded scratch piece that
+      // borrows the still unused ring, write with the lanes along the rows
+      float* scratch = reinterpret_cast<float*>(ring) + warp * (16 * 33);
+      static_assert(kPredictThreads / 32 * 16 * 33 * 4 <= 2 * kTreeBytes, "the pieces fit the ring");
       const int fpieces = (num_used + 31) / 32;
-      for (int piece = warp; piece < fpieces * (kTileThreads / 32); piece += kTileThreads / 32) {
+      for (int piece = warp; piece < fpieces * (tile_rows / 16); piece += kPredictThreads / 32) {
         const int fp = piece % fpieces, rp = piece / fpieces;
         const int j = fp * 32 + lane;
         const int col = j < num_used ? used[j] : -1;
-#pragma unroll 8
-        for (int k = 0; k < 32; ++k) {
-          const int r = row0 + rp * 32 + k;
-          float v = (col >= 0 && r < nrow) ? ToF<T>(data[static_cast<size_t>(r) * ncol + col]) : 0.f;
+#pragma unroll
+        for (int k = 0; k < 16; ++k) {
+          const int rr = row0 + rp * 16 + k;
+          float v = (col >= 0 && rr < nrow) ? ToF<T>(data[static_cast<size_t>(rr) * ncol + col]) : 0.f;
           if (PLAIN && isnan(v)) v = 0.f;
           scratch[k * 33 + lane] = v;
         }
         __syncwarp();
-#pragma unroll 8
-        for (int k = 0; k < 32; ++k) {
-          const int jj = fp * 32 + k;
-          if (jj < num_used) rows_s[jj * kTileThreads + rp * 32 + lane] = scratch[lane * 33 + k];
+#pragma unroll
+        for (int k = 0; k < 32; k += 2) {
+          const int jj = fp * 32 + k + (lane >> 4);
+          if (jj < num_used) rows_s[jj * tile_rows + rp * 16 + (lane & 15)] = scratch[(lane & 15) * 33 + k + (lane >> 4)];
         }
         __syncwarp();
       }
@@ -101,62 +121,60 @@ PredictTiledKernel(const unsigned char* __restrict__ blob, const ChunkDesc* __re
       if (c < num_chunks) {
         const ChunkDesc d = chunks[c];
         const uint4* src = reinterpret_cast<const uint4*>(blob + d.offset);
-        uint4* dst = reinterpret_cast<uint4*>(ring + (c & 1) * kChunkBytes);
-        for (int i = tid; i < d.bytes / 16; i += kTileThreads) __pipeline_memcpy_async(dst + i, src + i, 16);
+        uint4* dst = reinterpret_cast<uint4*>(ring + (c & 1) * chunk_bytes);
+        for (int i = tid; i < d.bytes / 16; i += kPredictThreads) __pipeline_memcpy_async(dst + i, src + i, 16);
       }
       __pipeline_commit();
+    };
+    // the slices' sums of one class, added in slice order; all threads of the block
+    auto finish_class = [&](int cls, double acc) {
+      sums[tid] = acc;
+      __syncthreads();
+      if (slice == 0 && row < nrow) {
+        double t = sums[r];
+        for (int k = 1; k < slices; ++k) t += sums[(k << log_rows) + r];
+        out[static_cast<size_t>(cls) * nrow + row] = static_cast<float>(t * inv_avg);
+      }
+      __syncthreads();
     };
     fetch(0);
     double acc = 0.0;   // a forest of a thousand trees summed in float would drift from the host's double sums
     int cur_cls = num_chunks > 0 ? chunks[0].cls : 0;
-    const float* my = rows_s + tid;
     for (int c = 0; c < num_chunks; ++c) {
       fetch(c + 1);
       __pipeline_wait_prior(1);
       __syncthreads();
       const ChunkDesc d = chunks[c];
-      if (!LEAF && d.cls != cur_cls) {
-        if (row < nrow) out[static_cast<size_t>(cur_cls) * nrow + row] = static_cast<float>(acc * inv_avg);
-        acc = 0.0; cur_cls = d.cls;
-      }
-      const unsigned char* buf = ring + (c & 1) * kChunkBytes;
-      const int* roots = reinterpret_cast<const int*>(buf);          // [ntrees] node index of every tree's root, then the nodes
-      const PackedNode* nodes = reinterpret_cast<const PackedNode*>(buf + ((d.ntrees * 4 + 15) & ~15));
-      for (int t = 0; t < d.ntrees; t += kWalks) {
-        // kWalks walks in flight, written without branches so that their shared-memory loads overlap: a walk that has
-        // reached its leaf (or has no tree) re-reads its own node and feature slot 0 until the others are done
-        int at[kWalks], base[kWalks]; PackedNode nd[kWalks]; bool live[kWalks];
-        bool any = false;
+      if (!LEAF && d.cls != cur_cls) { finish_class(cur_cls, acc); acc = 0.0; cur_cls = d.cls; }
+      const unsigned int buf = (c & 1) * chunk_bytes;
+      const int* roots = reinterpret_cast<const int*>(smem + buf + d.roots);   // [ntrees] chunk offset of every tree's root
+      for (int t = slice * kWalks; t < d.ntrees; t += slices * kWalks) {
+        PackedNode nd[kWalks];
 #pragma unroll
-        for (int q = 0; q < kWalks; ++q) {
-          const bool has = t + q < d.ntrees;
-          base[q] = has ? roots[t + q] : 0;
-          at[q] = base[q];
-          nd[q] = nodes[at[q]];
-          live[q] = has && (nd[q].meta & 0xFFFFu) != kLeafSlot;
-          any = any || live[q];
-        }
-        while (any) {
+        for (int q = 0; q < kWalks; ++q) nd[q] = *reinterpret_cast<const PackedNode*>(smem + buf + roots[min(t + q, d.ntrees - 1)]);   // past the last tree: walked again, not counted
+        auto step = [&]() {
           float v[kWalks];
 #pragma unroll
-          for (int q = 0; q < kWalks; ++q) v[q] = my[(live[q] ? (nd[q].meta & 0xFFFFu) : 0u) * kTileThreads];
+          for (int q = 0; q < kWalks; ++q) v[q] = *reinterpret_cast<const float*>(smem + (((nd[q].meta >> slot_shift) & slot_mask) | row_bytes));
 #pragma unroll
           for (int q = 0; q < kWalks; ++q) {
-            const int next = base[q] + static_cast<int>((nd[q].meta >> 16) & 0x1FFFu) + (GoLeft<PLAIN>(v[q], nd[q].value, nd[q].meta) ? 0 : 1);
-            at[q] = live[q] ? next : at[q];
+            unsigned int next = (nd[q].meta & kChildMask) | buf;
+            // a leaf stays where it is: -infinity goes left, and its left child is itself
+            if (!GoLeft<PLAIN>(v[q], nd[q].value, nd[q].meta)) next += 8u;
+            nd[q] = *reinterpret_cast<const PackedNode*>(smem + next);
           }
-          any = false;
+        };
+        for (;;) {
+          unsigned int all = nd[0].meta;
 #pragma unroll
-          for (int q = 0; q < kWalks; ++q) {
-            nd[q] = nodes[at[q]];
-            live[q] = live[q] && (nd[q].meta & 0xFFFFu) != kLeafSlot;
-            any = any || live[q];
-          }
+          for (int q = 1; q < kWalks; ++q) all &= nd[q].meta;
+          if ((all & (kLeafType << 1)) == (kLeafType << 1)) break;   // every walk is at a leaf
+          step(); step();
         }
 #pragma unroll
         for (int q = 0; q < kWalks; ++q) {
           if (t + q < d.ntrees) {
-            if (LEAF) { if (row < nrow) out_leaf[static_cast<size_t>(row) * trees_total + d.first_tree + (t + q) * num_class] = static_cast<int>((nd[q].meta >> 16) & 0x1FFFu); }
+            if (LEAF) { if (row < nrow) reinterpret_cast<int*>(out)[static_cast<size_t>(row) * trees_total + d.first_tree + (t + q) * num_class] = __float_as_int(nd[q].value); }
             else acc += static_cast<double>(nd[q].value);
           }
         }
@@ -164,41 +182,44 @@ PredictTiledKernel(const unsigned char* __restrict__ blob, const ChunkDesc* __re
       __syncthreads();   // everyone is done with this buffer before the fetch after next refills it
     }
     __pipeline_wait_prior(0);
-    if (!LEAF && num_chunks > 0 && row < nrow) out[static_cast<size_t>(cur_cls) * nrow + row] = static_cast<float>(acc * inv_avg);
+    if (!LEAF && num_chunks > 0) finish_class(cur_cls, acc);
   }
 }
 
-// Nodes of one tree in sibling-adjacent order: root first, then every split's two children next to each other.
-bool PackTree(const Tree& T, const std::vector<int>& slot_of_feature, std::vector<PackedNode>* out) {
+// Nodes of one tree in sibling-adjacent order, root first, then every split's two children next to each other, placed at
+// byte `base` of their chunk. slot_base: slot of the tile's first feature row; leaf_slot: slot of the row of -infinity.
+bool PackTree(const Tree& T, const std::vector<int>& slot_of_feature, int slot_base, int leaf_slot, bool leaf_index, int base, std::vector<PackedNode>* out,
+              std::vector<std::pair<int, int>>* queue) {
   const int L = T.num_leaves;
-  if (L > 4096) return false;
-  out->clear();
-  if (L <= 1) { PackedNode nd; nd.value = static_cast<float>(T.leaf_value[0]); nd.meta = kLeafSlot; out->push_back(nd); return true; }
-  out->resize(2 * L - 1);
-  // queue of (host node id, packed position); host ids: >= 0 split, < 0 leaf ~id
-  std::vector<std::pair<int, int>> queue; queue.reserve(2 * L);
-  queue.emplace_back(0, 0);
-  int next_free = 1;
-  for (size_t qi = 0; qi < queue.size(); ++qi) {
-    const int id = queue[qi].first, pos = queue[qi].second;
+  out->resize(std::max(1, 2 * L - 1));
+  auto offset = [&](int pos) { return static_cast<unsigned int>(base + pos * static_cast<int>(sizeof(PackedNode))); };
+  auto leaf_node = [&](int leaf, int pos) {
     PackedNode nd;
-    if (id < 0) {
-      const int leaf = ~id;
-      nd.value = static_cast<float>(T.leaf_value[leaf]); nd.meta = kLeafSlot | (static_cast<unsigned int>(leaf) << 16);
-    } else {
-      if (T.decision_type[id] & kCategoricalMask) return false;
-      float thr = static_cast<float>(T.threshold[id]);
-      // keep "v <= threshold" exact for float inputs: round the double threshold DOWN to float
-      if (static_cast<double>(thr) > T.threshold[id]) thr = std::nextafterf(thr, -std::numeric_limits<float>::infinity());
-      const int slot = slot_of_feature[T.split_feature[id]];
-      const int left_pos = next_free; next_free += 2;
-      nd.value = thr;
-      nd.meta = static_cast<unsigned int>(slot) | (static_cast<unsigned int>(left_pos) << 16) | ((T.decision_type[id] & kDefaultLeftMask) ? (1u << 29) : 0u) |
-                (static_cast<unsigned int>(Tree::MissingTypeOf(T.decision_type[id])) << 30);
-      queue.emplace_back(T.left_child[id], left_pos);
-      queue.emplace_back(T.right_child[id], left_pos + 1);
-    }
+    if (leaf_index) std::memcpy(&nd.value, &leaf, sizeof(int)); else nd.value = static_cast<float>(T.leaf_value[leaf]);
+    nd.meta = (static_cast<unsigned int>(leaf_slot) << 16) | offset(pos) | (kLeafType << 1);
+    return nd;
+  };
+  if (!leaf_index) for (int l = 0; l < std::max(1, L); ++l) if (std::isnan(T.leaf_value[l])) return false;   // a leaf holds its place by -infinity <= value
+  if (L <= 1) { (*out)[0] = leaf_node(0, 0); return true; }
+  // queue of (host node id, packed position); host ids: >= 0 split, < 0 leaf ~id
+  queue->clear();
+  queue->emplace_back(0, 0);
+  int next_free = 1;
+  for (size_t qi = 0; qi < queue->size(); ++qi) {
+    const int id = (*queue)[qi].first, pos = (*queue)[qi].second;
+    if (id < 0) { (*out)[pos] = leaf_node(~id, pos); continue; }
+    if (T.decision_type[id] & kCategoricalMask) return false;
+    float thr = static_cast<float>(T.threshold[id]);
+    // keep "v <= threshold" exact for float inputs: round the double threshold DOWN to float
+    if (static_cast<double>(thr) > T.threshold[id]) thr = std::nextafterf(thr, -std::numeric_limits<float>::infinity());
+    const int left_pos = next_free; next_free += 2;
+    PackedNode nd;
+    nd.value = thr;
+    nd.meta = (static_cast<unsigned int>(slot_base + slot_of_feature[T.split_feature[id]]) << 16) | offset(left_pos) |
+              (static_cast<unsigned int>(Tree::MissingTypeOf(T.decision_type[id])) << 1) | ((T.decision_type[id] & kDefaultLeftMask) ? 1u : 0u);
     (*out)[pos] = nd;
+    queue->emplace_back(T.left_child[id], left_pos);
+    queue->emplace_back(T.right_child[id], left_pos + 1);
   }
   return true;
 }
@@ -227,35 +248,47 @@ bool DevicePredictTiled(const GBDT* gbdt, const void* device_data, int dtype, in
   }
   std::vector<int> used;
   for (size_t f = 0; f < slot_of_feature.size(); ++f) if (slot_of_feature[f] == 0) { slot_of_feature[f] = static_cast<int>(used.size()); used.push_back(static_cast<int>(f)); }
-  if (used.size() >= kLeafSlot) return false;
   if (used.empty()) used.push_back(0);
-  const size_t smem = 2 * static_cast<size_t>(kChunkBytes) + used.size() * kTileThreads * sizeof(float);
-  if (smem > 220 * 1024) return false;
-  // chunks: trees of one class in iteration order, as many as fit a ring buffer
+  const int nu = static_cast<int>(used.size());
+  // leaf indices have no general kernel to fall back to: the widest forest is the one of a 256-row tile beside two chunks
+  if (leaf_index && 2 * kTreeBytes + nu * kMaxTileRows * 4 > kPredictSmem) return false;
+  int dev = 0, sms = 0; FB_CUDA(cudaGetDevice(&dev)); FB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  // The tile: as many rows as fit beside two chunks (the forest streams through the ring once per tile), but no more than
+  // leave every SM a tile; the threads that rows do not take walk other trees.
+  auto smem_of = [&](int log_rows, int chunk) { return 2 * static_cast<size_t>(chunk) + (static_cast<size_t>(nu + 1) << log_rows) * 4 + kPredictThreads * sizeof(double); };
+  int log_rows = 8;
+  while (log_rows > 5 && (smem_of(log_rows, kTreeBytes) > kPredictSmem || ((nrow + (1 << log_rows) - 1) >> log_rows) < sms)) --log_rows;
+  if (smem_of(log_rows, kTreeBytes) > kPredictSmem) return false;
+  const int chunk_bytes = smem_of(log_rows, 2 * kTreeBytes) <= kPredictSmem ? 2 * kTreeBytes : kTreeBytes;   // more trees per barrier where there is room
+  const size_t smem = smem_of(log_rows, chunk_bytes);
+  const int slot_base = (2 * chunk_bytes) >> (log_rows + 2);   // the tile's rows start behind the ring
+  if (slot_base + nu > 0xFFFF) return false;
+  // chunks: trees of one class in iteration order, as many as fit a ring buffer; the root words behind the nodes
   std::vector<unsigned char> blob; std::vector<ChunkDesc> chunks;
-  std::vector<PackedNode> packed;
+  std::vector<PackedNode> packed, nodes; std::vector<std::pair<int, int>> queue; std::vector<int> roots;
   for (int cls = 0; cls < K; ++cls) {
-    std::vector<int> roots; std::vector<PackedNode> nodes; int first = -1;
+    int first = -1;
     auto close = [&]() {
       if (roots.empty()) return;
-      ChunkDesc d; d.offset = static_cast<long long>(blob.size()); d.ntrees = static_cast<int>(roots.size()); d.cls = cls; d.first_tree = first;
-      const size_t head = (roots.size() * 4 + 15) & ~static_cast<size_t>(15);
-      const size_t bytes = (head + nodes.size() * sizeof(PackedNode) + 15) & ~static_cast<size_t>(15);
+      ChunkDesc d; d.offset = static_cast<long long>(blob.size()); d.ntrees = static_cast<int>(roots.size()); d.cls = cls; d.first_tree = first; d.pad = 0;
+      d.roots = static_cast<int>(nodes.size() * sizeof(PackedNode));
+      const size_t bytes = (d.roots + roots.size() * 4 + 15) & ~static_cast<size_t>(15);
       d.bytes = static_cast<int>(bytes);
       blob.resize(blob.size() + bytes, 0);
-      memcpy(blob.data() + d.offset, roots.data(), roots.size() * 4);
-      memcpy(blob.data() + d.offset + head, nodes.data(), nodes.size() * sizeof(PackedNode));
+      memcpy(blob.data() + d.offset, nodes.data(), nodes.size() * sizeof(PackedNode));
+      memcpy(blob.data() + d.offset + d.roots, roots.data(), roots.size() * 4);
       chunks.push_back(d); roots.clear(); nodes.clear(); first = -1;
     };
     for (int t = cls; t < num_trees; t += K) {
-      if (!PackTree(*gbdt->models_[first_tree + t], slot_of_feature, &packed)) return false;
-      const size_t need = (((roots.size() + 1) * 4 + 15) & ~static_cast<size_t>(15)) + (nodes.size() + packed.size()) * sizeof(PackedNode) + 16;
-      if (need > static_cast<size_t>(kChunkBytes)) {
-        close();
-        if (((4 + 15) & ~15) + packed.size() * sizeof(PackedNode) + 16 > static_cast<size_t>(kChunkBytes)) return false;   // a single tree larger than a buffer
-      }
+      const Tree& T = *gbdt->models_[first_tree + t];
+      const size_t tree_nodes = std::max(1, 2 * T.num_leaves - 1);
+      if (T.num_leaves > 4096 || tree_nodes * sizeof(PackedNode) + 32 > static_cast<size_t>(kTreeBytes)) return false;   // a single tree larger than a buffer
+      const size_t need = (nodes.size() + tree_nodes) * sizeof(PackedNode) + (roots.size() + 1) * 4 + 16;
+      if (need > static_cast<size_t>(chunk_bytes)) close();
+      const int base = static_cast<int>(nodes.size() * sizeof(PackedNode));
+      if (!PackTree(T, slot_of_feature, slot_base, slot_base + nu, leaf_index, base, &packed, &queue)) return false;
       if (first < 0) first = t;
-      roots.push_back(static_cast<int>(nodes.size()));
+      roots.push_back(base);
       nodes.insert(nodes.end(), packed.begin(), packed.end());
     }
     close();
@@ -263,16 +296,15 @@ bool DevicePredictTiled(const GBDT* gbdt, const void* device_data, int dtype, in
   if (chunks.empty()) return false;
   DevBuf<unsigned char> d_blob; DevBuf<ChunkDesc> d_chunks; DevBuf<int> d_used;
   d_blob.Upload(blob, s); d_chunks.Upload(chunks, s); d_used.Upload(used, s);
-  int dev = 0, sms = 0; FB_CUDA(cudaGetDevice(&dev)); FB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  const int tiles = (nrow + kTileThreads - 1) / kTileThreads;
+  const int tiles = (nrow + (1 << log_rows) - 1) >> log_rows;
   const int grid = std::min(tiles, sms);
-  const int nc = static_cast<int>(chunks.size()), nu = static_cast<int>(used.size());
+  const int nc = static_cast<int>(chunks.size());
 #define FB_TILED_P(T, LEAF, PLAIN)                                                                                                 \
   {                                                                                                                                \
     static bool attr = false;                                                                                                      \
-    if (!attr) { FB_CUDA(cudaFuncSetAttribute(PredictTiledKernel<T, LEAF, PLAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024)); attr = true; } \
-    PredictTiledKernel<T, LEAF, PLAIN><<<grid, kTileThreads, smem, s>>>(d_blob.get(), d_chunks.get(), nc, d_used.get(), nu, static_cast<const T*>(device_data), nrow, ncol, \
-                                                                        row_major ? 1 : 0, K, num_trees, inv_avg, out_device, reinterpret_cast<int*>(out_device));          \
+    if (!attr) { FB_CUDA(cudaFuncSetAttribute(PredictTiledKernel<T, LEAF, PLAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPredictSmem)); attr = true; } \
+    PredictTiledKernel<T, LEAF, PLAIN><<<grid, kPredictThreads, smem, s>>>(d_blob.get(), d_chunks.get(), nc, chunk_bytes, d_used.get(), nu, static_cast<const T*>(device_data), nrow, ncol, \
+                                                                           row_major ? 1 : 0, log_rows, K, num_trees, inv_avg, out_device);   \
   }
 #define FB_TILED(T, LEAF) { if (plain) FB_TILED_P(T, LEAF, true) else FB_TILED_P(T, LEAF, false) }
   if (leaf_index) {
