@@ -10,7 +10,7 @@ constexpr int kCtrlThreads = 256;
 
 __global__ void __launch_bounds__(kCtrlThreads) LevelControllerKernel(CtrlArgs a) {
   __shared__ CtrlShared S;
-  ControllerBody<kCtrlThreads>(a, S);
+  ControllerBody(a, S, false);
 }
 
 // One thread sets up everything a tree starts from, from the device-side gradient sums (no host round trip

@@ -15,14 +15,17 @@ namespace fb {
 
 constexpr int kCtrlMaxLeaves = 1024;
 
-// Shared-memory working set of the controller (the caller provides it: a kernel's static shared memory).
+// Shared-memory working set of the controller (the caller provides it).
 struct CtrlShared {
-  int leaf[kCtrlMaxLeaves];            // candidate leaves, later the chosen leaves in ascending order
-  double gain[kCtrlMaxLeaves / 2];     // scratch view: the chosen leaves as ints
-  int order[kCtrlMaxLeaves];
-  int chunks[kCtrlMaxLeaves / 2 + 1], blocks[kCtrlMaxLeaves / 2 + 1];
+  int leaf[kCtrlMaxLeaves];               // candidate leaves
+  double gain[kCtrlMaxLeaves];            // and their gains
+  int rank[kCtrlMaxLeaves];               // leaf-wise growth: evaluated nodes before the candidate (kNotKept: beyond the budget)
+  int chosen[kCtrlMaxLeaves];             // chosen leaves in ascending order
+  int chunks[kCtrlMaxLeaves], blocks[kCtrlMaxLeaves];   // their exclusive prefixes
+  unsigned int kept[kCtrlMaxLeaves / 32];               // chosen leaves as a bit set
+  int kept_before[kCtrlMaxLeaves / 32];                 // chosen leaves before each word
   double first[2 * kCtrlMaxLeaves + 2];   // leaf-wise growth: first order-key step of every evaluated node
-  int ncand, nkeep;
+  int ncand, nkeep, total_chunks, total_blocks;
 };
 
 // A record that another block of the SAME launch may have written a moment ago: read through L2, in 8-byte pieces
@@ -45,108 +48,116 @@ __device__ inline T LoadWords(const T* p) {
   return v;
 }
 
-// Call with all T threads of one block. Reads the level record `a.cur`, writes the next level's into `a.nxt`.
-template <int T>
-__device__ inline void ControllerBody(const CtrlArgs& a, CtrlShared& S) {
-  int num_eval_out = LoadWords(&a.cur->num_eval);
+// Call with all threads of one block (whole warps). Reads the level record `a.cur`, writes the next level's into `a.nxt`.
+// listed: the caller has filled S.leaf / S.gain / S.ncand with the frontier leaves that have a usable split.
+__device__ inline void ControllerBody(const CtrlArgs& a, CtrlShared& S, bool listed) {
+  constexpr int kNotKept = 0x7fffffff;
+  const int T = blockDim.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = T >> 5;
   // the level record is read whole before anything is written: `cur` and `nxt` may be the same object
   const LevelCtrl c0 = LoadWords(a.cur);
+  int num_eval_out = c0.num_eval;
   LevelCtrl* c = a.nxt;
-  const int nfront = c0.done ? 0 : c0.frontier_count;
-  if (threadIdx.x == 0) { S.ncand = 0; S.nkeep = 0; }
-  __syncthreads();
-  // 1. candidates: frontier leaves with a usable split
-  for (int i = threadIdx.x; i < nfront; i += T) {
-    const int l = a.frontier[i];
-    const SplitRecord b = LoadWords(a.best + l);
-    if (b.feature >= 0 && b.gain > 0.0) { const int p = atomicAdd(&S.ncand, 1); S.leaf[p] = l; }
+  if (!listed) {
+    if (threadIdx.x == 0) S.ncand = 0;
+    __syncthreads();
+    // 1. candidates: frontier leaves with a usable split
+    const int nfront = c0.done ? 0 : c0.frontier_count;
+    for (int i = threadIdx.x; i < nfront; i += T) {
+      const int l = a.frontier[i];
+      const int feature = LoadWords(&a.best[l].feature); const double gain = LoadWords(&a.best[l].gain);
+      if (feature >= 0 && gain > 0.0) { const int p = atomicAdd(&S.ncand, 1); S.leaf[p] = l; S.gain[p] = gain; }
+    }
   }
+  for (int w = threadIdx.x; w < kCtrlMaxLeaves / 32; w += T) S.kept[w] = 0u;
   __syncthreads();
   const int ncand = S.ncand;
   const int budget = a.max_leaves - c0.num_leaves;
   if (a.leafwise_budget > 0) {
     // 2'. leaf-wise: record the order keys of the newly evaluated nodes, then keep the candidates with fewer than
     //     leafwise_budget evaluated nodes strictly before them; if the growth cap binds, the best of those by rank
-    const int base_eval = c0.num_eval;
-    for (int i = threadIdx.x; i < ncand; i += T) {
-      const int li = S.leaf[i];
-      LeafwiseChildKey(LoadWords(a.leaves + li).pkey, LoadWords(a.best + li).gain, a.eval_key + static_cast<size_t>(base_eval + i) * 4);
-    }
-    __syncthreads();
-    const int total = base_eval + ncand;
+    const int base_eval = c0.num_eval, total = base_eval + ncand;
     // first key step of every evaluated node in shared memory: it decides nearly every comparison
-    for (int j = threadIdx.x; j < total; j += T) S.first[j] = a.eval_key[static_cast<size_t>(j) * 4];
+    for (int j = threadIdx.x; j < base_eval; j += T) S.first[j] = a.eval_key[static_cast<size_t>(j) * 4];
+    for (int i = threadIdx.x; i < ncand; i += T) {
+      double key[4];
+      LeafwiseChildKey(LoadWords(a.leaves + S.leaf[i]).pkey, S.gain[i], key);
+      for (int k = 0; k < 4; ++k) a.eval_key[static_cast<size_t>(base_eval + i) * 4 + k] = key[k];
+      S.first[base_eval + i] = key[0];
+    }
     __syncthreads();
-    {
-      // one warp per candidate, the lanes stride over the evaluated nodes
-      const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-      for (int i = warp; i < ncand; i += T / 32) {
-        double ki[4]; for (int k = 0; k < 4; ++k) ki[k] = a.eval_key[static_cast<size_t>(base_eval + i) * 4 + k];
-        int cnt = 0;
-        for (int j = lane; j < total; j += 32) {
-          const double pj = S.first[j];
-          bool before = pj > ki[0];
-          if (pj == ki[0]) before = LeafwiseKeyBefore(a.eval_key + static_cast<size_t>(j) * 4, ki);
-          cnt += before ? 1 : 0;
-        }
-        for (int o = 16; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-        if (lane == 0) S.order[i] = cnt < a.leafwise_budget ? cnt : 0x7fffffff;
+    // one warp per candidate, the lanes stride over the evaluated nodes
+    for (int i = warp; i < ncand; i += warps) {
+      double ki[4]; for (int k = 0; k < 4; ++k) ki[k] = a.eval_key[static_cast<size_t>(base_eval + i) * 4 + k];
+      int cnt = 0;
+#pragma unroll 4
+      for (int j = lane; j < total; j += 32) {
+        const double pj = S.first[j];
+        bool before = pj > ki[0];
+        if (pj == ki[0]) before = LeafwiseKeyBefore(a.eval_key + static_cast<size_t>(j) * 4, ki);
+        cnt += before ? 1 : 0;
       }
+      cnt = __reduce_add_sync(0xffffffffu, cnt);
+      if (lane == 0) S.rank[i] = cnt < a.leafwise_budget ? cnt : kNotKept;
     }
-    __syncthreads();
-    unsigned int keep_bits = 0;   // this thread's decisions, one bit per stride step (written back after all ranks were read)
-    for (int i = threadIdx.x, step = 0; i < ncand; i += T, ++step) {
-      const int ri = S.order[i];
-      bool keep = ri != 0x7fffffff;
-      if (keep) { int better = 0; for (int j = 0; j < ncand; ++j) better += (S.order[j] < ri) || (S.order[j] == ri && S.leaf[j] < S.leaf[i]); keep = better < budget; }
-      if (keep) keep_bits |= 1u << step;
-    }
-    __syncthreads();
-    for (int i = threadIdx.x, step = 0; i < ncand; i += T, ++step) S.order[i] = (keep_bits >> step) & 1u;
     num_eval_out = total;
-  } else {
-  // 2. rank by (gain desc, leaf asc) when the budget binds; 3. order the kept ones by leaf id
-  for (int i = threadIdx.x; i < ncand; i += T) {
-    const int li = S.leaf[i]; const double gi = LoadWords(&a.best[li].gain);
-    bool keep = true;
-    if (ncand > budget) {
-      int better = 0;
-      for (int j = 0; j < ncand; ++j) { const int lj = S.leaf[j]; const double gj = LoadWords(&a.best[lj].gain); better += (gj > gi) || (gj == gi && lj < li); }
-      keep = better < budget;
-    }
-    S.order[i] = keep ? 1 : 0;
+    __syncthreads();
   }
+  // 2. rank when the budget binds: by gain (ties: lower leaf id), or by the leaf-wise rank; the kept ones as a bit set
+  for (int i = warp; i < ncand; i += warps) {
+    const int li = S.leaf[i];
+    bool keep = a.leafwise_budget <= 0 || S.rank[i] != kNotKept;
+    if (keep && ncand > budget) {
+      int better = 0;
+      for (int j = lane; j < ncand; j += 32) {
+        const int lj = S.leaf[j];
+        if (a.leafwise_budget > 0) better += (S.rank[j] < S.rank[i]) || (S.rank[j] == S.rank[i] && lj < li);
+        else better += (S.gain[j] > S.gain[i]) || (S.gain[j] == S.gain[i] && lj < li);
+      }
+      keep = __reduce_add_sync(0xffffffffu, better) < budget;
+    }
+    if (keep && lane == 0) atomicOr(&S.kept[li >> 5], 1u << (li & 31));
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < ncand; i += T) {
-    if (!S.order[i]) continue;
-    const int li = S.leaf[i];
-    int pos = 0;
-    for (int j = 0; j < ncand; ++j) pos += (S.order[j] && S.leaf[j] < li);
-    // chosen leaves go to the upper half of a scratch view: write after everyone has read
-    reinterpret_cast<int*>(S.gain)[pos] = li;
-    atomicAdd(&S.nkeep, 1);
+  // 3. the kept leaves by leaf id
+  if (warp == 0) {
+    static_assert(kCtrlMaxLeaves / 32 == 32, "a word per lane");
+    const int n = __popc(S.kept[lane]);
+    int incl = n;
+    for (int o = 1; o < 32; o <<= 1) { const int y = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += y; }
+    S.kept_before[lane] = incl - n;
+    if (lane == 31) S.nkeep = incl;
   }
   __syncthreads();
   const int NS = S.nkeep;
-  int* chosen = reinterpret_cast<int*>(S.gain);
-  // 4. local allotments (chunks of the partition, blocks of the construct) and their prefixes
-  for (int s = threadIdx.x; s < NS; s += T) {
-    const int cnt = LoadWords(&a.leaves[chosen[s]].count);
-    S.chunks[s] = max(1, (cnt + kPartChunk - 1) / kPartChunk);   // at least one: the chunk block of a split also sets up its children
+  for (int i = threadIdx.x; i < ncand; i += T) {
+    const int li = S.leaf[i];
+    const unsigned int word = S.kept[li >> 5], bit = 1u << (li & 31);
+    if (!(word & bit)) continue;
+    const int s = S.kept_before[li >> 5] + __popc(word & (bit - 1u));
+    S.chosen[s] = li;
+    // 4. local allotments: chunks of the partition (at least one: the chunk block of a split also sets up its children), blocks of the construct
+    const int cnt = LoadWords(&a.leaves[li].count);
+    S.chunks[s] = max(1, (cnt + kPartChunk - 1) / kPartChunk);
     S.blocks[s] = max(1, (cnt + a.rows_per_block - 1) / a.rows_per_block);
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
+  if (warp == 0) {
     int ac = 0, ab = 0;
-    for (int s = 0; s < NS; ++s) { const int t = S.chunks[s]; S.chunks[s] = ac; ac += t; const int u = S.blocks[s]; S.blocks[s] = ab; ab += u; }
-    S.chunks[NS] = ac; S.blocks[NS] = ab;
+    for (int s0 = 0; s0 < NS; s0 += 32) {
+      const int s = s0 + lane;
+      const int vc = s < NS ? S.chunks[s] : 0, vb = s < NS ? S.blocks[s] : 0;
+      int ic = vc, ib = vb;
+      for (int o = 1; o < 32; o <<= 1) { const int yc = __shfl_up_sync(0xffffffffu, ic, o), yb = __shfl_up_sync(0xffffffffu, ib, o); if (lane >= o) { ic += yc; ib += yb; } }
+      if (s < NS) { S.chunks[s] = ac + ic - vc; S.blocks[s] = ab + ib - vb; }
+      ac += __shfl_sync(0xffffffffu, ic, 31); ab += __shfl_sync(0xffffffffu, ib, 31);
+    }
+    if (lane == 0) { S.total_chunks = ac; S.total_blocks = ab; }
   }
   __syncthreads();
   // 5. descriptors
   const int base_leaf = c0.num_leaves, base_slot = c0.next_slot, base_journal = c0.journal_count;
   for (int s = threadIdx.x; s < NS; s += T) {
-    const int l = chosen[s];
+    const int l = S.chosen[s];
     const int right = base_leaf + s;
     const LeafInfo P = LoadWords(a.leaves + l);
     const SplitRecord b = LoadWords(a.best + l);
@@ -155,7 +166,7 @@ __device__ inline void ControllerBody(const CtrlArgs& a, CtrlShared& S) {
     q.leaf = l; q.right_leaf = right; q.begin = P.begin; q.count = P.count; q.buffer = P.buffer; q.group = m.group; q.bundled = m.bundled; q.group_offset = m.group_offset;
     q.num_bin = m.num_bin; q.most_freq_bin = m.most_freq_bin; q.threshold = b.threshold; q.default_left = b.default_left; q.missing_type = m.missing_type;
     q.default_bin = m.default_bin; q.is_categorical = b.is_categorical; for (int w = 0; w < 8; ++w) q.cat_bitset[w] = b.cat_bitset[w];
-    q.chunk_begin = S.chunks[s]; q.num_chunks = S.chunks[s + 1] - S.chunks[s]; q.pad_[0] = q.pad_[1] = 0;
+    q.chunk_begin = S.chunks[s]; q.num_chunks = max(1, (P.count + kPartChunk - 1) / kPartChunk); q.pad_[0] = q.pad_[1] = 0;
     q.owner = a.bin_owner != nullptr ? a.bin_owner[m.hist_offset] : 0;
     a.splits[s] = q;
     ChildInit ci;
@@ -164,7 +175,7 @@ __device__ inline void ControllerBody(const CtrlArgs& a, CtrlShared& S) {
     ci.left_slot = ci.smaller_is_left ? fresh : P.hist_slot; ci.right_slot = ci.smaller_is_left ? P.hist_slot : fresh;
     ci.left_g = b.left_g; ci.left_h = b.left_h; ci.right_g = b.right_g; ci.right_h = b.right_h; ci.left_out = b.left_out; ci.right_out = b.right_out;
     ci.left_gi = b.left_gi; ci.left_hi = b.left_hi; ci.right_gi = P.sum_gi - b.left_gi; ci.right_hi = P.sum_hi - b.left_hi;
-    ci.hist_block_begin = S.blocks[s]; ci.hist_num_blocks = S.blocks[s + 1] - S.blocks[s];
+    ci.hist_block_begin = S.blocks[s]; ci.hist_num_blocks = max(1, (P.count + a.rows_per_block - 1) / a.rows_per_block);
     ci.monotone = b.monotone; ci.pad_ = 0; LeafwiseChildKey(P.pkey, b.gain, ci.pkey);
     a.child_init[s] = ci;
     FindChild fl, fr;
@@ -175,16 +186,15 @@ __device__ inline void ControllerBody(const CtrlArgs& a, CtrlShared& S) {
     j.begin = P.begin; j.count = P.count; j.buffer = P.buffer; j.depth = P.depth;
     a.journal[base_journal + s] = j;
   }
-  __syncthreads();
   // 6. new frontier (children in split order) and the level record
-  for (int s = threadIdx.x; s < NS; s += T) { a.frontier[2 * s] = chosen[s]; a.frontier[2 * s + 1] = base_leaf + s; }
+  for (int s = threadIdx.x; s < NS; s += T) { a.frontier[2 * s] = S.chosen[s]; a.frontier[2 * s + 1] = base_leaf + s; }
   if (threadIdx.x == 0) {
     LevelCtrl o = c0;
     o.num_leaves = base_leaf + NS; o.next_slot = base_slot + NS; o.journal_count = base_journal + NS; o.level = c0.level + 1; o.num_eval = num_eval_out;
     // A level that uses up the leaf budget ends the tree: its children are partitioned (the score update and the
     // leaf counts need their windows) but neither constructed nor searched.
     const bool last = base_leaf + NS >= a.max_leaves;
-    o.num_splits = NS; o.num_children = 2 * NS; o.total_chunks = S.chunks[NS]; o.total_blocks = last ? 0 : S.blocks[NS];
+    o.num_splits = NS; o.num_children = 2 * NS; o.total_chunks = S.total_chunks; o.total_blocks = last ? 0 : S.total_blocks;
     o.skip_search = last ? 1 : 0;
     o.frontier_count = last ? 0 : 2 * NS;
     if (NS == 0) o.done = 1; else o.pad0 = o.level;   // pad0: last level that applied a split

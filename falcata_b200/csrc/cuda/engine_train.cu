@@ -137,7 +137,9 @@ Tree* CudaEngine::TrainTree(int class_id, int tree_index) {
   col_sampler_.ResetByTree(tree_index);
   // features searched on this rank this tree (owned, sampled, numerical) and the rest of the owned ones
   std::vector<int> feats, subs;
-  for (int f : owned_features_) { if (col_sampler_.used_by_tree()[f]) feats.push_back(f); else subs.push_back(f); }
+  // (one rank: the histograms of features outside the sample are read by forced splits only)
+  const bool keep_unsampled = world_ > 1 || !forced_.empty();
+  for (int f : owned_features_) { if (col_sampler_.used_by_tree()[f]) feats.push_back(f); else if (keep_unsampled) subs.push_back(f); }
   features_.Upload(feats, stream_); sub_features_.Upload(subs, stream_);
   const int NF = static_cast<int>(feats.size()), NS = static_cast<int>(subs.size());
   std::vector<int> feats_all, subs_all;   // voting: the local pass searches every sampled feature, owned or not
@@ -374,14 +376,14 @@ Tree* CudaEngine::TrainTree(int class_id, int tree_index) {
     PartArgs pa = PartArgs();
     pa.rows = dd_->rows.get(); pa.row_stride = dd_->row_stride; pa.idx[0] = idx_[0].get(); pa.idx[1] = idx_[1].get();
     pa.cols = dd_->cols.size() ? dd_->cols.get() : nullptr; pa.col_stride = n_;
-    pa.splits = ca.splits; pa.num_splits = max_splits; pa.total_chunks = n_ / kPartChunk + max_splits; pa.bits = bits_.get(); pa.chunk_left = chunk_left_.get();
+    pa.splits = ca.splits; pa.bits = bits_.get(); pa.chunk_left = chunk_left_.get();
     pa.split_left_total = split_left_total_.get(); pa.leaves = leaves_.get(); pa.child_init = ca.child_init; pa.hist_tasks = hist_tasks_.get(); pa.rows_per_block = rpb;
     pa.world = dp ? world_ : 1;
     pa.chunk_words = one_launch_part ? chunk_words_.get() : nullptr;
     if (dp) for (int r = 0; r < world_; ++r) pa.peer_counts[r] = fabric_->Ptr<int>(r, off_counts_) + static_cast<size_t>(rank_) * NL;
     if (feature_parallel_) SetupBitmapBroadcast(&pa);
-    ha.identity_root = 0; ha.rows_per_block = rpb; ha.num_tasks = max_splits; ha.total_blocks = n_ / rpb + max_splits;
-    fa.children = ca.children; fa.num_children = 2 * max_splits;
+    ha.identity_root = 0; ha.rows_per_block = rpb;
+    fa.children = ca.children;
     int level = 0;   // index of the last level enqueued (0 = root)
     auto enqueue_level = [&]() {
       ++level;
@@ -390,6 +392,10 @@ Tree* CudaEngine::TrainTree(int class_id, int tree_index) {
       if (!fused_tail) LaunchLevelController(ca, stream_);
       else { ca.cur = lc; ca.nxt = ctrl_.get() + ((level + 1) & 1); }
       pa.ctrl = lc; ha.ctrl = lc; fa.ctrl = lc;
+      // grids are upper bounds: level k has at most 2^(k - 1) splits
+      const int splits = level < 20 ? std::min(max_splits, 1 << (level - 1)) : max_splits;
+      pa.num_splits = splits; pa.total_chunks = n_ / kPartChunk + splits;
+      ha.num_tasks = splits; ha.total_blocks = n_ / rpb + splits; fa.num_children = 2 * splits;
       if (num_sets_ > 0) LaunchPathBits(lc, journal_.get(), dd_->feature_meta.get(), path_bits_.get(), path_words_, max_splits, stream_);
       if (feature_parallel_) { pa.bc_sig.epoch = fabric_->NextEpoch(); pa.bc_wait.epoch = pa.bc_sig.epoch; }
       clock_.Begin(st_part_, stream_);

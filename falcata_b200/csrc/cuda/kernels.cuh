@@ -112,6 +112,7 @@ struct CandLite {      // best threshold of one (child, feature)
   double gain; int feature; int threshold; int default_left; int left_cnt;
   long long left_gi, left_hi; double left_g, left_h;
   int is_categorical, num_cat_bins; uint32_t cat_bitset[8];   // categorical: the bins that go left
+  int real, pad;                                              // real index of the feature (ties between features go to the lower one)
 };
 
 struct FindArgs {
@@ -124,7 +125,7 @@ struct FindArgs {
   const LeafInfo* leaves;
   const float* scales;                            // quantized: (g_scale, h_scale) of this tree
   SplitParams params;
-  CandLite* cand;                                 // [num_children x num_features]
+  CandLite* cand;                                 // [num_children x num_features]; fused tail on one rank: [num_children x search blocks of a child]
   SplitRecord* best;                              // [leaf]
   int quant;
   int tree_index; unsigned int extra_seed;        // extra_trees: key of the per-(tree, leaf, feature) threshold draw

@@ -7,16 +7,19 @@
 // two produce bit-identical gains.
 #include "controller.cuh"
 
+#include <type_traits>
+
 namespace fb {
 
 namespace {
 
-constexpr int kFindThreads = 256;
-constexpr int kWarpsPerBlock = kFindThreads / 32;
+constexpr int kFindThreads = 512;   // at most: a warp per (child, feature); fewer for few features
 
-struct Acc {   // prefix accumulator of one lane
-  long long gi, hi; double gd, hd; int c;
-};
+// Shared memory of a search block: the warps' staged bins (numerical features) or scratch (categorical ones) and the warps'
+// best candidates; then, in the last block of a level, the tail's working set in the same bytes.
+extern __shared__ __align__(16) unsigned char find_smem[];
+constexpr int kStagedBins = 256 + 32;   // 32 lane runs of up to 8 bins, one entry apart (8- and 16-byte accesses without bank conflicts)
+template <bool QUANT> constexpr int kStagedBytes = kStagedBins * (QUANT ? 8 : 16);
 
 // Where the bins of one (child, feature) come from.
 //  one rank  : child slot (smaller child: constructed there; larger child: still the parent) and,
@@ -64,6 +67,13 @@ __device__ inline int ChildGlobalCount(const FindArgs& a, const FindChild& ch, i
   return ch.is_left ? lsum : ch.parent_global - lsum;
 }
 
+__device__ inline CandLite NoCandidate() {
+  CandLite c; c.gain = -1.0 / 0.0; c.feature = -1; c.threshold = 0; c.default_left = 1; c.left_cnt = 0; c.left_gi = c.left_hi = 0; c.left_g = c.left_h = 0;
+  c.is_categorical = 0; c.num_cat_bins = 0; for (int w = 0; w < 8; ++w) c.cat_bitset[w] = 0;
+  c.real = -1; c.pad = 0;
+  return c;
+}
+
 // Categorical search of one (child, feature) by one warp. The bins are staged in shared memory (and
 // written back where the child's histogram is formed on the fly); the sort by g / (h + cat_smooth) is a
 // rank count over all lanes (stable: ties keep bin order); the two directional scans run on lane 0 in
@@ -73,9 +83,8 @@ constexpr int kCatMaxBins = 256;
 struct CatScratch { double g[kCatMaxBins], h[kCatMaxBins]; long long gi[kCatMaxBins], hi[kCatMaxBins]; unsigned char order[kCatMaxBins]; };
 
 template <bool QUANT>
-__device__ void ScanCategoricalWarp(const FindArgs& a, const BinSrc& src, char* child, bool write_back, const FeatureMeta& m, const LeafInfo& leaf, int f, int fi,
-                                    int lane, int warp) {
-  extern __shared__ __align__(16) unsigned char find_smem[];
+__device__ void ScanCategoricalWarp(const FindArgs& a, const BinSrc& src, char* child, bool write_back, const FeatureMeta& m, const LeafInfo& leaf, int f,
+                                    int lane, int warp, CandLite* out) {
   CatScratch& S = reinterpret_cast<CatScratch*>(find_smem)[warp];
   const int nb = m.num_bin;
   const int nstored = m.bundled ? nb - 1 : nb;
@@ -135,8 +144,7 @@ __device__ void ScanCategoricalWarp(const FindArgs& a, const BinSrc& src, char* 
   }
   __syncwarp();
   if (lane != 0) return;
-  CandLite c; c.gain = -1.0 / 0.0; c.feature = -1; c.threshold = 0; c.default_left = 0; c.left_cnt = 0; c.left_gi = c.left_hi = 0; c.left_g = c.left_h = 0;
-  c.is_categorical = 1; c.num_cat_bins = 0; for (int w = 0; w < 8; ++w) c.cat_bitset[w] = 0;
+  CandLite c = NoCandidate(); c.default_left = 0; c.is_categorical = 1;
   double best_gain = -1.0 / 0.0; int best_dir = -1, best_k = -1;
   if (onehot) {
     for (int b = 1; b < nb; ++b) {
@@ -166,17 +174,19 @@ __device__ void ScanCategoricalWarp(const FindArgs& a, const BinSrc& src, char* 
       c.num_cat_bins = best_k + 1;
     }
   }
-  if (best_k >= 0 && best_gain != -1.0 / 0.0) { c.gain = FB_MUL(best_gain, static_cast<double>(m.penalty)); c.feature = f; }
-  a.cand[static_cast<size_t>(blockIdx.x) * a.num_features + fi] = c;
+  if (best_k >= 0 && best_gain != -1.0 / 0.0) { c.gain = FB_MUL(best_gain, static_cast<double>(m.penalty)); c.feature = f; c.real = m.real_index; }
+  *out = c;
 }
 
-// The search of one (child, feature) by one warp; warps of a block work on different features of the same child and
-// leave independently (only warp-level synchronisation inside).
+// The search of one (child, feature) by one warp; warps of a block work on different features of the same child. The
+// warp's candidate (or "none") goes to `out` - shared or global memory.
+//
+// What bounds it is latency: a level of 16 children is a handful of blocks. The feature's bins come in with all loads in
+// flight at once and are staged in shared memory; a lane then owns a run of 1, 2, 4 or 8 consecutive bins, so the warp makes
+// ONE prefix scan over the lane totals (integer sums: on the packed 64-bit word) instead of one per 32 bins.
 template <bool QUANT>
-__device__ void FindSplitsWarp(const FindArgs& a) {
+__device__ void FindSplitsWarp(const FindArgs& a, int fi, CandLite* out) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int fi = blockIdx.y * kWarpsPerBlock + warp;
-  if (fi >= a.num_features + a.num_sub_features) return;
   const bool search = fi < a.num_features;
   const int f = search ? a.features[fi] : a.sub_features[fi - a.num_features];
   const FindChild ch = a.children[blockIdx.x];
@@ -204,22 +214,14 @@ __device__ void FindSplitsWarp(const FindArgs& a) {
   const int stage_task = vote_global ? static_cast<int>(blockIdx.x) : ch.task;
   src.stage = world > 1 ? static_cast<const char*>(a.stage) + (static_cast<long long>(stage_task) * a.slot_stride + base) * esz : nullptr;
   if (vote_global && (!search || a.voted[static_cast<size_t>(blockIdx.x) * a.voted_stride + f] == 0)) {
-    if (search && lane == 0) {
-      CandLite c; c.gain = -1.0 / 0.0; c.feature = -1; c.threshold = 0; c.default_left = 1; c.left_cnt = 0; c.left_gi = c.left_hi = 0; c.left_g = c.left_h = 0;
-      c.is_categorical = 0; c.num_cat_bins = 0; for (int w = 0; w < 8; ++w) c.cat_bitset[w] = 0;
-      a.cand[static_cast<size_t>(blockIdx.x) * a.num_features + fi] = c;
-    }
+    if (search && lane == 0) *out = NoCandidate();
     return;
   }
 
   const bool node_masked = search && a.node_mask != nullptr && a.node_mask[static_cast<size_t>(blockIdx.x) * a.node_mask_stride + f] == 0;
-  if (node_masked && lane == 0) {
-    CandLite c; c.gain = -1.0 / 0.0; c.feature = -1; c.threshold = 0; c.default_left = 1; c.left_cnt = 0; c.left_gi = c.left_hi = 0; c.left_g = c.left_h = 0;
-    c.is_categorical = 0; c.num_cat_bins = 0; for (int w = 0; w < 8; ++w) c.cat_bitset[w] = 0;
-    a.cand[static_cast<size_t>(blockIdx.x) * a.num_features + fi] = c;
-  }
+  if (node_masked && lane == 0) *out = NoCandidate();
   if (search && !node_masked && m.bin_type != 0) {
-    ScanCategoricalWarp<QUANT>(a, src, child, write_back, m, leaf, f, fi, lane, warp);
+    ScanCategoricalWarp<QUANT>(a, src, child, write_back, m, leaf, f, lane, warp, out);
     return;
   }
   if (!search || node_masked) {
@@ -246,95 +248,129 @@ __device__ void FindSplitsWarp(const FindArgs& a) {
   const int skip = two_pass ? (m.missing_type == 1 ? m.default_bin : nb - 1) : -1;
   const int mfb = m.bundled ? m.most_freq_bin : -1;
 
-  // pre-pass: the un-stored most-frequent bin of a bundled feature = leaf total - sum of stored bins
-  long long mfb_gi = 0, mfb_hi = 0; double mfb_gd = 0, mfb_hd = 0;
-  if (m.bundled) {
-    long long sgi = 0, shi = 0; double sgd = 0, shd = 0;
-    for (int j = lane; j < nstored; j += 32) {
-      long long gi = 0, hi = 0; double gd = 0, hd = 0; hist_q_t rq; double2 rd;
-      LoadBin<QUANT>(src, j, &gi, &hi, &gd, &hd, &rq, &rd);
-      sgi += gi; shi += hi; sgd += gd; shd += hd;
+  // stage: bin b of the feature at entry b + (b >> per_log), lane l owns bins [l << per_log, (l + 1) << per_log)
+  using Bin = std::conditional_t<QUANT, hist_q_t, double2>;
+  Bin* bins = reinterpret_cast<Bin*>(find_smem + warp * (a.has_categorical ? static_cast<int>(sizeof(CatScratch)) : kStagedBytes<QUANT>));
+  const int per_log = nb <= 32 ? 0 : (nb <= 64 ? 1 : (nb <= 128 ? 2 : 3)), pad_shift = per_log == 0 ? 31 : per_log;
+  auto entry = [&](int b) { return b + (b >> pad_shift); };
+  hist_q_t sum_q = 0; double2 sum_d = make_double2(0.0, 0.0);   // all stored bins of a bundled feature
+  for (int b0 = 0; b0 < nb; b0 += 128) {
+    Bin v[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int b = b0 + 32 * k + lane;
+      long long gi, hi; double gd, hd; hist_q_t rq = 0; double2 rd = make_double2(0.0, 0.0);
+      if (b < nb && b != mfb) LoadBin<QUANT>(src, (mfb >= 0 && b > mfb) ? b - 1 : b, &gi, &hi, &gd, &hd, &rq, &rd);
+      if constexpr (QUANT) v[k] = rq; else v[k] = rd;
     }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int b = b0 + 32 * k + lane;
+      if (b >= nb) continue;
+      bins[entry(b)] = v[k];
+      if (write_back && b != mfb) reinterpret_cast<Bin*>(child)[(mfb >= 0 && b > mfb) ? b - 1 : b] = v[k];
+      if constexpr (QUANT) sum_q += v[k]; else { sum_d.x += v[k].x; sum_d.y += v[k].y; }
+    }
+  }
+  if (mfb >= 0) {
+    // the un-stored most-frequent bin of a bundled feature = leaf total - sum of stored bins
     for (int o = 16; o > 0; o >>= 1) {
-      sgi += __shfl_xor_sync(0xffffffffu, sgi, o); shi += __shfl_xor_sync(0xffffffffu, shi, o);
-      sgd += __shfl_xor_sync(0xffffffffu, sgd, o); shd += __shfl_xor_sync(0xffffffffu, shd, o);
+      if constexpr (QUANT) sum_q += __shfl_xor_sync(0xffffffffu, sum_q, o);
+      else { sum_d.x += __shfl_xor_sync(0xffffffffu, sum_d.x, o); sum_d.y += __shfl_xor_sync(0xffffffffu, sum_d.y, o); }
     }
-    mfb_gi = L.sum_gi - sgi; mfb_hi = L.sum_hi - shi; mfb_gd = L.sum_g - sgd; mfb_hd = L.sum_h - shd;
+    if (lane == 0) { if constexpr (QUANT) bins[entry(mfb)] = HistQPack(L.sum_gi, L.sum_hi) - sum_q; else bins[entry(mfb)] = make_double2(L.sum_g - sum_d.x, L.sum_h - sum_d.y); }
   }
+  __syncwarp();
+  auto real_h = [&](const Bin& v) -> double { if constexpr (QUANT) return FB_MUL(static_cast<double>(HistQHess(v)), L.h_scale); else return v.y; };
   // mass of the missing-value bin (kept out of the prefix, added on the left in pass 0)
-  long long Mgi = 0, Mhi = 0; double Mgd = 0, Mhd = 0; int Mc = 0;
-  if (skip >= 0) {
-    if (skip == mfb) { Mgi = mfb_gi; Mhi = mfb_hi; Mgd = mfb_gd; Mhd = mfb_hd; }
-    else { hist_q_t rq; double2 rd; LoadBin<QUANT>(src, (mfb >= 0 && skip > mfb) ? skip - 1 : skip, &Mgi, &Mhi, &Mgd, &Mhd, &rq, &rd); }
-    const double hreal = QUANT ? FB_MUL(static_cast<double>(Mhi), L.h_scale) : Mhd;
-    Mc = BinCountEstimate(hreal, L.cnt_factor);
+  Bin M; if constexpr (QUANT) M = 0; else M = make_double2(0.0, 0.0);
+  int Mc = 0;
+  if (skip >= 0) { M = bins[entry(skip)]; Mc = BinCountEstimate(real_h(M), L.cnt_factor); }
+
+  // exclusive prefix of this lane's run: lane totals, one warp scan
+  const int run0 = lane << per_log, run1 = min(nb, run0 + (1 << per_log));
+  Bin acc; if constexpr (QUANT) acc = 0; else acc = make_double2(0.0, 0.0);
+  int c = 0;
+  for (int b = run0; b < run1; ++b) {
+    if (b == skip) continue;
+    const Bin v = bins[entry(b)];
+    if constexpr (QUANT) acc += v; else { acc.x += v.x; acc.y += v.y; }
+    c += BinCountEstimate(real_h(v), L.cnt_factor);
   }
+  for (int o = 1; o < 32; o <<= 1) {
+    if constexpr (QUANT) { const hist_q_t t = __shfl_up_sync(0xffffffffu, acc, o); if (lane >= o) acc += t; }
+    else { const double tx = __shfl_up_sync(0xffffffffu, acc.x, o), ty = __shfl_up_sync(0xffffffffu, acc.y, o); if (lane >= o) { acc.x += tx; acc.y += ty; } }
+    const int tc = __shfl_up_sync(0xffffffffu, c, o); if (lane >= o) c += tc;
+  }
+  if constexpr (QUANT) acc = __shfl_up_sync(0xffffffffu, acc, 1);
+  else { acc.x = __shfl_up_sync(0xffffffffu, acc.x, 1); acc.y = __shfl_up_sync(0xffffffffu, acc.y, 1); }
+  c = __shfl_up_sync(0xffffffffu, c, 1);
+  if (lane == 0) { if constexpr (QUANT) acc = 0; else acc = make_double2(0.0, 0.0); c = 0; }
 
   double best_gain = -1.0 / 0.0; int best_rank = 1 << 30, best_t = 0, best_pass = 0, best_lc = 0;
   long long best_lgi = 0, best_lhi = 0; double best_lg = 0, best_lh = 0;
   const int rand_t = a.params.extra_trees ? ExtraTreesThreshold(a.extra_seed, a.tree_index, ch.leaf, m.real_index, nb) : -1;
-  Acc carry; carry.gi = carry.hi = 0; carry.gd = carry.hd = 0; carry.c = 0;
-  for (int b0 = 0; b0 < nb; b0 += 32) {
-    const int b = b0 + lane;
-    long long gi = 0, hi = 0; double gd = 0, hd = 0; int c = 0;
-    if (b < nb) {
-      if (b == mfb) { gi = mfb_gi; hi = mfb_hi; gd = mfb_gd; hd = mfb_hd; }
-      else {
-        const int j = (mfb >= 0 && b > mfb) ? b - 1 : b;
-        hist_q_t rq; double2 rd;
-        LoadBin<QUANT>(src, j, &gi, &hi, &gd, &hd, &rq, &rd);
-        if (write_back) { if (QUANT) reinterpret_cast<hist_q_t*>(child)[j] = rq; else reinterpret_cast<double2*>(child)[j] = rd; }
-      }
-      if (b == skip) { gi = hi = 0; gd = hd = 0; }
-      else { const double hreal = QUANT ? FB_MUL(static_cast<double>(hi), L.h_scale) : hd; c = BinCountEstimate(hreal, L.cnt_factor); }
+  for (int b = run0; b < run1; ++b) {
+    if (b != skip) {
+      const Bin v = bins[entry(b)];
+      if constexpr (QUANT) acc += v; else { acc.x += v.x; acc.y += v.y; }
+      c += BinCountEstimate(real_h(v), L.cnt_factor);
     }
-    // inclusive warp scan
-    for (int o = 1; o < 32; o <<= 1) {
-      const long long tg = __shfl_up_sync(0xffffffffu, gi, o), th = __shfl_up_sync(0xffffffffu, hi, o);
-      const double dg = __shfl_up_sync(0xffffffffu, gd, o), dh = __shfl_up_sync(0xffffffffu, hd, o);
-      const int tc = __shfl_up_sync(0xffffffffu, c, o);
-      if (lane >= o) { gi += tg; hi += th; gd += dg; hd += dh; c += tc; }
-    }
-    gi += carry.gi; hi += carry.hi; gd += carry.gd; hd += carry.hd; c += carry.c;
-    if (b <= nb - 2 && (rand_t < 0 || b == rand_t)) {
-      for (int pass = 0; pass < (two_pass ? 2 : 1); ++pass) {
-        if (b == skip && pass == 1 && m.missing_type == 1) continue;
-        long long lgi = gi, lhi = hi; int lc = c; double lg, lh;
-        const bool addm = pass == 0 && skip >= 0;
-        if (addm) { lgi += Mgi; lhi += Mhi; lc += Mc; }
-        if (QUANT) { lg = FB_MUL(static_cast<double>(lgi), L.g_scale); lh = FB_MUL(static_cast<double>(lhi), L.h_scale); }
-        else { lg = gd + (addm ? Mgd : 0.0); lh = hd + (addm ? Mhd : 0.0); }
-        double lo, ro;
-        const double gain = EvalCandidate(lg, lh, lc, L, a.params, m.monotone, &lo, &ro);
-        if (gain == -1.0 / 0.0) continue;
-        const int rank = ScanRank(pass, b, nb);
-        if (gain > best_gain || (gain == best_gain && rank < best_rank)) {
-          best_gain = gain; best_rank = rank; best_t = b; best_pass = pass; best_lc = lc; best_lgi = lgi; best_lhi = lhi; best_lg = lg; best_lh = lh;
-        }
+    if (b > nb - 2 || (rand_t >= 0 && b != rand_t)) continue;
+    for (int pass = 0; pass < (two_pass ? 2 : 1); ++pass) {
+      if (b == skip && pass == 1 && m.missing_type == 1) continue;
+      const bool addm = pass == 0 && skip >= 0;
+      const int lc = c + (addm ? Mc : 0);
+      long long lgi = 0, lhi = 0; double lg, lh;
+      if constexpr (QUANT) {
+        const hist_q_t w = addm ? acc + M : acc;
+        lgi = HistQGrad(w); lhi = HistQHess(w);
+        lg = FB_MUL(static_cast<double>(lgi), L.g_scale); lh = FB_MUL(static_cast<double>(lhi), L.h_scale);
+      } else { lg = acc.x + (addm ? M.x : 0.0); lh = acc.y + (addm ? M.y : 0.0); }
+      double lo, ro;
+      const double gain = EvalCandidate(lg, lh, lc, L, a.params, m.monotone, &lo, &ro);
+      if (gain == -1.0 / 0.0) continue;
+      const int rank = ScanRank(pass, b, nb);
+      if (gain > best_gain || (gain == best_gain && rank < best_rank)) {
+        best_gain = gain; best_rank = rank; best_t = b; best_pass = pass; best_lc = lc; best_lgi = lgi; best_lhi = lhi; best_lg = lg; best_lh = lh;
       }
     }
-    carry.gi = __shfl_sync(0xffffffffu, gi, 31); carry.hi = __shfl_sync(0xffffffffu, hi, 31);
-    carry.gd = __shfl_sync(0xffffffffu, gd, 31); carry.hd = __shfl_sync(0xffffffffu, hd, 31); carry.c = __shfl_sync(0xffffffffu, c, 31);
   }
-  // warp argmax: larger gain, then lower scan rank
+  // warp argmax: larger gain, then lower scan rank (ranks differ between candidates); the winner's lane writes
+  double top_gain = best_gain; int top_rank = best_rank;
   for (int o = 16; o > 0; o >>= 1) {
-    const double og = __shfl_xor_sync(0xffffffffu, best_gain, o); const int orank = __shfl_xor_sync(0xffffffffu, best_rank, o);
-    const int ot = __shfl_xor_sync(0xffffffffu, best_t, o), op = __shfl_xor_sync(0xffffffffu, best_pass, o), olc = __shfl_xor_sync(0xffffffffu, best_lc, o);
-    const long long ogi = __shfl_xor_sync(0xffffffffu, best_lgi, o), ohi = __shfl_xor_sync(0xffffffffu, best_lhi, o);
-    const double olg = __shfl_xor_sync(0xffffffffu, best_lg, o), olh = __shfl_xor_sync(0xffffffffu, best_lh, o);
-    if (og > best_gain || (og == best_gain && orank < best_rank)) {
-      best_gain = og; best_rank = orank; best_t = ot; best_pass = op; best_lc = olc; best_lgi = ogi; best_lhi = ohi; best_lg = olg; best_lh = olh;
-    }
+    const double og = __shfl_xor_sync(0xffffffffu, top_gain, o); const int orank = __shfl_xor_sync(0xffffffffu, top_rank, o);
+    if (og > top_gain || (og == top_gain && orank < top_rank)) { top_gain = og; top_rank = orank; }
   }
-  if (lane == 0) {
-    CandLite c;
-    const bool ok = best_gain != -1.0 / 0.0;
-    c.gain = ok ? FB_MUL(best_gain, static_cast<double>(m.penalty)) : best_gain;
-    c.feature = ok ? f : -1; c.threshold = best_t; c.default_left = best_pass == 0 ? 1 : 0; c.left_cnt = best_lc;
-    c.left_gi = best_lgi; c.left_hi = best_lhi; c.left_g = best_lg; c.left_h = best_lh;
-    c.is_categorical = 0; c.num_cat_bins = 0; for (int w = 0; w < 8; ++w) c.cat_bitset[w] = 0;
-    a.cand[static_cast<size_t>(blockIdx.x) * a.num_features + fi] = c;
+  if (top_rank == 1 << 30) { if (lane == 0) *out = NoCandidate(); }
+  else if (best_rank == top_rank) {
+    CandLite r = NoCandidate();
+    r.gain = FB_MUL(best_gain, static_cast<double>(m.penalty)); r.feature = f; r.real = m.real_index;
+    r.threshold = best_t; r.default_left = best_pass == 0 ? 1 : 0; r.left_cnt = best_lc;
+    r.left_gi = best_lgi; r.left_hi = best_lhi; r.left_g = best_lg; r.left_h = best_lh;
+    *out = r;
   }
+}
+
+// The split record of a child from its best candidate (null: none).
+__device__ inline SplitRecord MakeRecord(const FindArgs& a, const LeafInfo& leaf, const CandLite* best) {
+  SplitRecord r; InitSplitRecord(&r);
+  const bool depth_ok = a.params.max_depth <= 0 || leaf.depth < a.params.max_depth;
+  const bool size_ok = leaf.num_data_global >= 2 * a.params.min_data_in_leaf;
+  if (best != nullptr && depth_ok && size_ok) {
+    const CandLite c = LoadWords(best);
+    r.gain = c.gain; r.feature = c.feature; r.threshold = c.threshold; r.default_left = c.default_left;
+    if (a.params.cegb_split > 0.0) r.gain -= a.params.cegb_split * static_cast<double>(leaf.num_data_global);
+    r.left_g = c.left_g; r.left_h = c.left_h; r.right_g = FB_SUB(leaf.sum_g, c.left_g); r.right_h = FB_SUB(leaf.sum_h, c.left_h);
+    r.left_gi = c.left_gi; r.left_hi = c.left_hi; r.left_cnt = c.left_cnt; r.right_cnt = leaf.num_data_global - c.left_cnt;
+    r.monotone = c.is_categorical ? 0 : a.meta[c.feature].monotone;
+    r.is_categorical = c.is_categorical; r.num_cat_bins = c.num_cat_bins; for (int w = 0; w < 8; ++w) r.cat_bitset[w] = c.cat_bitset[w];
+    SplitParams p = a.params; if (c.is_categorical) p.lambda_l2 = FB_ADD(p.lambda_l2, a.params.cat_l2);
+    r.left_out = LeafOutput(r.left_g, FB_ADD(r.left_h, kEpsilon), p, r.left_cnt, leaf.output);
+    r.right_out = LeafOutput(r.right_g, FB_ADD(r.right_h, kEpsilon), p, r.right_cnt, leaf.output);
+    if (p.use_mc != 0) { r.left_out = ClampOutput(r.left_out, leaf.min_c, leaf.max_c); r.right_out = ClampOutput(r.right_out, leaf.min_c, leaf.max_c); }
+  }
+  return r;
 }
 
 // Per-leaf argmax over the searched features of one child -> SplitRecord (the CPU's tie order: higher gain, then
@@ -342,8 +378,9 @@ __device__ void FindSplitsWarp(const FindArgs& a) {
 // owns; it is stored into every rank's slot array. Call with all T threads of a block.
 struct ReduceShared { SplitRecord rec; double gain[kFindThreads]; int feat[kFindThreads], thr[kFindThreads], idx[kFindThreads]; };
 
-template <int T>
+// (a block of a power of two of threads, at most kFindThreads)
 __device__ inline void ReduceChildBody(const FindArgs& a, int child, ReduceShared& R) {
+  const int T = blockDim.x;
   const bool gather = a.wait_best.world > 1;   // data-parallel and feature-parallel both all-gather the rank-local best
   const FindChild ch = a.children[child];
   LeafInfo leaf = a.leaves[ch.leaf];
@@ -354,9 +391,8 @@ __device__ inline void ReduceChildBody(const FindArgs& a, int child, ReduceShare
   const bool searched = !(a.ctrl != nullptr && a.ctrl->skip_search);
   for (int k = threadIdx.x; searched && k < a.num_features; k += T) {
     const CandLite* cp = a.cand + static_cast<size_t>(child) * a.num_features + k;
-    const double gain = LoadWords(&cp->gain); const int feature = LoadWords(&cp->feature), threshold = LoadWords(&cp->threshold);
-    const int rf = feature >= 0 ? a.meta[feature].real_index : -1;
-    if (SplitBetter(gain, rf, threshold, bg, bf, bt)) { bg = gain; bf = rf; bt = threshold; bi = k; }
+    const double gain = LoadWords(&cp->gain); const int real = LoadWords(&cp->real), threshold = LoadWords(&cp->threshold);
+    if (SplitBetter(gain, real, threshold, bg, bf, bt)) { bg = gain; bf = real; bt = threshold; bi = k; }
   }
   R.gain[threadIdx.x] = bg; R.feat[threadIdx.x] = bf; R.thr[threadIdx.x] = bt; R.idx[threadIdx.x] = bi;
   __syncthreads();
@@ -367,22 +403,7 @@ __device__ inline void ReduceChildBody(const FindArgs& a, int child, ReduceShare
     __syncthreads();
   }
   if (threadIdx.x == 0) {
-    SplitRecord r; InitSplitRecord(&r);
-    const bool depth_ok = a.params.max_depth <= 0 || leaf.depth < a.params.max_depth;
-    const bool size_ok = leaf.num_data_global >= 2 * a.params.min_data_in_leaf;
-    if (R.idx[0] >= 0 && depth_ok && size_ok) {
-      const CandLite c = LoadWords(a.cand + static_cast<size_t>(child) * a.num_features + R.idx[0]);
-      r.gain = c.gain; r.feature = c.feature; r.threshold = c.threshold; r.default_left = c.default_left;
-      if (a.params.cegb_split > 0.0) r.gain -= a.params.cegb_split * static_cast<double>(leaf.num_data_global);
-      r.left_g = c.left_g; r.left_h = c.left_h; r.right_g = FB_SUB(leaf.sum_g, c.left_g); r.right_h = FB_SUB(leaf.sum_h, c.left_h);
-      r.left_gi = c.left_gi; r.left_hi = c.left_hi; r.left_cnt = c.left_cnt; r.right_cnt = leaf.num_data_global - c.left_cnt;
-      r.monotone = c.is_categorical ? 0 : a.meta[c.feature].monotone;
-      r.is_categorical = c.is_categorical; r.num_cat_bins = c.num_cat_bins; for (int w = 0; w < 8; ++w) r.cat_bitset[w] = c.cat_bitset[w];
-      SplitParams p = a.params; if (c.is_categorical) p.lambda_l2 = FB_ADD(p.lambda_l2, a.params.cat_l2);
-      r.left_out = LeafOutput(r.left_g, FB_ADD(r.left_h, kEpsilon), p, r.left_cnt, leaf.output);
-      r.right_out = LeafOutput(r.right_g, FB_ADD(r.right_h, kEpsilon), p, r.right_cnt, leaf.output);
-      if (p.use_mc != 0) { r.left_out = ClampOutput(r.left_out, leaf.min_c, leaf.max_c); r.right_out = ClampOutput(r.right_out, leaf.min_c, leaf.max_c); }
-    }
+    const SplitRecord r = MakeRecord(a, leaf, R.idx[0] >= 0 ? a.cand + static_cast<size_t>(child) * a.num_features + R.idx[0] : nullptr);
     if (gather) { R.rec = r; a.leaves_rw[ch.leaf].num_data_global = leaf.num_data_global; }
     else a.best[ch.leaf] = r;
   }
@@ -393,7 +414,7 @@ __device__ inline void ReduceChildBody(const FindArgs& a, int child, ReduceShare
     constexpr int kWords = sizeof(SplitRecord) / 4;
     for (int p = 0; p < a.wait_best.world; ++p) {
       unsigned int* dst = reinterpret_cast<unsigned int*>(a.peer_best[p] + ch.leaf);
-      for (int w = threadIdx.x; w < kWords; w += T) dst[w] = src[w];
+      for (int w = threadIdx.x; w < kWords; w += blockDim.x) dst[w] = src[w];
     }
   }
 }
@@ -416,15 +437,18 @@ __device__ inline void GatherChild(const FindArgs& a, int child) {
   a.best[ch.leaf] = best;
 }
 
+union TailShared { ReduceShared r; CtrlShared c; };
+
 template <bool QUANT>
-__global__ void __launch_bounds__(kFindThreads) FindSplitsKernel(FindArgs a, CtrlArgs ca) {
+__global__ void __launch_bounds__(kFindThreads, 2) FindSplitsKernel(FindArgs a, CtrlArgs ca) {
   __shared__ int s_last;
-  __shared__ union TailShared { ReduceShared r; CtrlShared c; } S;
+  __shared__ CandLite s_cand[kFindThreads / 32];
+  TailShared& S = *reinterpret_cast<TailShared*>(find_smem);   // used once the block's search is over
   const int nchildren = a.ctrl != nullptr ? a.ctrl->num_children : a.num_children;
   if (nchildren <= 0) {
     // A level past the end of the tree (levels are enqueued ahead): nothing to search, but the NEXT level's record must
     // still be written, or that level would run on the stale record its ring half holds from two levels ago.
-    if (a.fused_tail && a.run_controller && blockIdx.x == 0 && blockIdx.y == 0) ControllerBody<kFindThreads>(ca, S.c);
+    if (a.fused_tail && a.run_controller && blockIdx.x == 0 && blockIdx.y == 0) ControllerBody(ca, S.c, false);
     return;
   }
   if (static_cast<int>(blockIdx.x) >= nchildren) return;
@@ -432,12 +456,68 @@ __global__ void __launch_bounds__(kFindThreads) FindSplitsKernel(FindArgs a, Ctr
   // orders the peers' child counts (stored by their partition, before their construct) ahead of the per-leaf
   // argmax that follows, so it is taken even when the search itself is skipped.
   if (a.wait.world > 1) FabricWaitAll(a.wait);
-  // skip_search: the tree is complete, nothing was constructed for these children
-  if (!(a.ctrl != nullptr && a.ctrl->skip_search)) FindSplitsWarp<QUANT>(a);
+  const bool gather = a.wait_best.world > 1;
+  const bool block_cand = a.fused_tail && !gather;   // one candidate per block; otherwise one per feature
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+  const bool searched = !(a.ctrl != nullptr && a.ctrl->skip_search);   // otherwise the tree is complete, nothing was constructed for these children
+  const int fi = blockIdx.y * warps + warp;
+  if (searched) {
+    if (block_cand && fi >= a.num_features && lane == 0) s_cand[warp] = NoCandidate();
+    if (fi < a.num_features + a.num_sub_features)
+      FindSplitsWarp<QUANT>(a, fi, block_cand ? s_cand + warp : a.cand + static_cast<size_t>(blockIdx.x) * a.num_features + fi);
+  }
   if (!a.fused_tail) return;
-
-  // ---- fused tail, step 1: the last block of this child reduces the child's candidates ----
   __syncthreads();   // every warp's candidate is written
+
+  if (!gather) {
+    // ---- fused tail, one rank: the block's best candidate, then the last block of the level takes over ----
+    if (searched && warp == 0) {
+      int best = lane < warps ? lane : 0;
+      for (int o = 8; o > 0; o >>= 1) {
+        const int other = __shfl_xor_sync(0xffffffffu, best, o);
+        const CandLite& x = s_cand[other]; const CandLite& y = s_cand[best];
+        if (SplitBetter(x.gain, x.real, x.threshold, y.gain, y.real, y.threshold)) best = other;
+      }
+      best = __shfl_sync(0xffffffffu, best, 0);
+      static_assert(sizeof(CandLite) % 4 == 0 && sizeof(CandLite) / 4 <= 32, "a record is copied by one warp");
+      if (lane < static_cast<int>(sizeof(CandLite) / 4))
+        reinterpret_cast<unsigned int*>(a.cand + static_cast<size_t>(blockIdx.x) * gridDim.y + blockIdx.y)[lane] = reinterpret_cast<const unsigned int*>(s_cand + best)[lane];
+    }
+    if (warp == 0) {
+      __syncwarp();
+      if (lane == 0) {
+        __threadfence();
+        const unsigned int prev = atomicAdd(a.level_done, 1u);
+        s_last = (prev + 1 == static_cast<unsigned int>(nchildren) * gridDim.y) ? 1 : 0;
+        if (s_last) *a.level_done = 0;
+      }
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    if (threadIdx.x == 0) S.c.ncand = 0;
+    __syncthreads();
+    // one thread per child: best of its blocks' candidates -> record -> the controller's candidate list
+    for (int child = threadIdx.x; child < nchildren; child += blockDim.x) {
+      const FindChild ch = a.children[child];
+      const LeafInfo leaf = a.leaves[ch.leaf];
+      double bg = -1.0 / 0.0; int bf = -1, bt = 0; const CandLite* best = nullptr;
+      for (unsigned int k = 0; searched && k < gridDim.y; ++k) {
+        const CandLite* cp = a.cand + static_cast<size_t>(child) * gridDim.y + k;
+        const double gain = LoadWords(&cp->gain); const int real = LoadWords(&cp->real), threshold = LoadWords(&cp->threshold);
+        if (SplitBetter(gain, real, threshold, bg, bf, bt)) { bg = gain; bf = real; bt = threshold; best = cp; }
+      }
+      const SplitRecord r = MakeRecord(a, leaf, best);
+      a.best[ch.leaf] = r;
+      if (r.feature >= 0 && r.gain > 0.0) { const int p = atomicAdd(&S.c.ncand, 1); S.c.leaf[p] = ch.leaf; S.c.gain[p] = r.gain; }
+    }
+    __threadfence();
+    __syncthreads();
+    if (a.run_controller) ControllerBody(ca, S.c, true);
+    return;
+  }
+
+  // ---- fused tail, several ranks, step 1: the last block of this child reduces the child's candidates ----
   if (threadIdx.x == 0) {
     __threadfence();
     const unsigned int prev = atomicAdd(a.child_done + blockIdx.x, 1u);
@@ -447,35 +527,32 @@ __global__ void __launch_bounds__(kFindThreads) FindSplitsKernel(FindArgs a, Ctr
   __syncthreads();
   if (!s_last) return;
   __threadfence();
-  ReduceChildBody<kFindThreads>(a, blockIdx.x, S.r);
+  ReduceChildBody(a, blockIdx.x, S.r);
   // ---- step 2: the last reducer of the level takes over ----
-  const bool gather = a.wait_best.world > 1;
   __syncthreads();
   if (threadIdx.x == 0) {
-    if (gather) __threadfence_system(); else __threadfence();   // this block's record (peer stores included) is published before it is counted
+    __threadfence_system();   // this block's record (peer stores included) is published before it is counted
     const unsigned int prev = atomicAdd(a.level_done, 1u);
     s_last = (prev + 1 == static_cast<unsigned int>(nchildren)) ? 1 : 0;
     if (s_last) *a.level_done = 0;
   }
   __syncthreads();
   if (!s_last) return;
-  if (gather) {
-    // every child's record of this rank is on its way: raise "best published" on every peer, wait (bounded) for
-    // theirs, then take the argmax over ranks for every child
-    if (threadIdx.x == 0) { __threadfence_system(); for (int r = 0; r < a.sig.world; ++r) StoreFlagAfterFence(a.sig.peer_flag[r], a.sig.epoch); }
-    FabricWaitAll(a.wait_best);
-    for (int c = threadIdx.x; c < nchildren; c += kFindThreads) GatherChild(a, c);
-  }
+  // every child's record of this rank is on its way: raise "best published" on every peer, wait (bounded) for
+  // theirs, then take the argmax over ranks for every child
+  if (threadIdx.x == 0) { __threadfence_system(); for (int r = 0; r < a.sig.world; ++r) StoreFlagAfterFence(a.sig.peer_flag[r], a.sig.epoch); }
+  FabricWaitAll(a.wait_best);
+  for (int c = threadIdx.x; c < nchildren; c += blockDim.x) GatherChild(a, c);
   __threadfence();
   __syncthreads();
-  if (a.run_controller) ControllerBody<kFindThreads>(ca, S.c);
+  if (a.run_controller) ControllerBody(ca, S.c, false);
 }
 
 __global__ void __launch_bounds__(128) ReduceBestKernel(FindArgs a) {
   const bool gather = a.wait_best.world > 1;
   if (static_cast<int>(blockIdx.x) >= (a.ctrl != nullptr ? a.ctrl->num_children : a.num_children)) { if (gather) FabricSignalDone(a.sig, gridDim.x); return; }
   __shared__ ReduceShared R;
-  ReduceChildBody<128>(a, blockIdx.x, R);
+  ReduceChildBody(a, blockIdx.x, R);
   if (gather) FabricSignalDone(a.sig, gridDim.x, true);
 }
 
@@ -499,17 +576,20 @@ void LaunchFindSplits(const FindArgs& a, cudaStream_t s, const CtrlArgs* tail_ct
   const int nf = a.num_features + a.num_sub_features;
   if (nf <= 0 && !a.fused_tail) return;
   if (a.fused_tail && a.run_controller && (tail_ctrl == nullptr || tail_ctrl->max_leaves > kCtrlMaxLeaves)) Log::Fatal("The fused level controller handles up to %d leaves", kCtrlMaxLeaves);
-  dim3 grid(a.num_children, std::max(1, (nf + kWarpsPerBlock - 1) / kWarpsPerBlock));
-  // categorical features stage their bins in shared memory, one scratch per warp
-  const size_t sm = a.has_categorical ? sizeof(CatScratch) * kWarpsPerBlock : 0;
+  const int warps = nf <= 8 ? 8 : kFindThreads / 32;   // a power of two; the tail's block works on up to 1024 leaves
+  dim3 grid(a.num_children, std::max(1, (nf + warps - 1) / warps));
+  size_t sm = static_cast<size_t>(warps) * (a.has_categorical ? std::max<size_t>(sizeof(CatScratch), a.quant ? kStagedBytes<true> : kStagedBytes<false>) : (a.quant ? kStagedBytes<true> : kStagedBytes<false>));
+  if (a.fused_tail) sm = std::max(sm, sizeof(TailShared));
   static bool attr = false;
-  if (sm > 16 * 1024 && !attr) {   // together with the tail's static shared memory the default limit is passed early
-    FB_CUDA(cudaFuncSetAttribute(FindSplitsKernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sm)));
-    FB_CUDA(cudaFuncSetAttribute(FindSplitsKernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sm)));
+  if (!attr) {
+    constexpr int kMaxSmem = static_cast<int>(std::max(sizeof(CatScratch) * (kFindThreads / 32), sizeof(TailShared)));
+    static_assert(kMaxSmem <= 220 * 1024 && sizeof(CatScratch) >= kStagedBytes<false>, "a block of categorical warps fits an SM");
+    FB_CUDA(cudaFuncSetAttribute(FindSplitsKernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem));
+    FB_CUDA(cudaFuncSetAttribute(FindSplitsKernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem));
     attr = true;
   }
   const CtrlArgs ca = tail_ctrl != nullptr ? *tail_ctrl : CtrlArgs();
-  if (a.quant) FindSplitsKernel<true><<<grid, kFindThreads, sm, s>>>(a, ca); else FindSplitsKernel<false><<<grid, kFindThreads, sm, s>>>(a, ca);
+  if (a.quant) FindSplitsKernel<true><<<grid, warps * 32, sm, s>>>(a, ca); else FindSplitsKernel<false><<<grid, warps * 32, sm, s>>>(a, ca);
   FB_LAUNCHED(); FB_KERNEL_CHECK();
 }
 
