@@ -85,7 +85,8 @@ struct DeviceDataset {
   int row_stride = 0;
   int gh_offset = -1;
   DevBuf<uint8_t> rows;
-  DevBuf<uint8_t> cols;        // optional column-major copy [num_groups x num_data]: the row partition reads ONE column
+  DevBuf<uint8_t> cols;        // optional column-major copy [num_groups x col_stride()]: the row partition reads ONE column
+  long long col_stride() const { return (static_cast<long long>(num_data) + 15) / 16 * 16; }   // whole 16-byte pieces
   DevBuf<float> label, weight;
   DevBuf<int> query_boundaries;
   int num_queries = 0;

@@ -236,7 +236,7 @@ Tree* CudaEngine::TrainTree(int class_id, int tree_index) {
       if (glist != compact_list_ || p4 != compact_p4_) {   // the view depends on the list only: trees that sample the same groups reuse it
         compact_groups_.Upload(glist, stream_); compact_start_.Upload(gstart, stream_); compact_count_.Upload(gcount, stream_);
         if (compact_rows_.size() < static_cast<size_t>(n_) * cstride) compact_rows_.Alloc(static_cast<size_t>(n_) * cstride);
-        LaunchCompactGather(dd_->cols.get(), n_, n_, compact_groups_.get(), nlist, compact_rows_.get(), cstride, stream_, p4);
+        LaunchCompactGather(dd_->cols.get(), dd_->col_stride(), n_, compact_groups_.get(), nlist, compact_rows_.get(), cstride, stream_, p4);
         FB_CUDA(cudaStreamSynchronize(stream_));   // the host lists above go out of scope
         compact_list_ = glist; compact_p4_ = p4;
       }
@@ -375,7 +375,7 @@ Tree* CudaEngine::TrainTree(int class_id, int tree_index) {
     FB_CUDA(cudaMemcpyAsync(h_root_.get(), leaves_.get(), sizeof(LeafInfo), cudaMemcpyDeviceToHost, stream_));   // the root record, before any split rewrites leaf 0
     PartArgs pa = PartArgs();
     pa.rows = dd_->rows.get(); pa.row_stride = dd_->row_stride; pa.idx[0] = idx_[0].get(); pa.idx[1] = idx_[1].get();
-    pa.cols = dd_->cols.size() ? dd_->cols.get() : nullptr; pa.col_stride = n_;
+    pa.cols = dd_->cols.size() ? dd_->cols.get() : nullptr; pa.col_stride = dd_->col_stride();
     pa.splits = ca.splits; pa.bits = bits_.get(); pa.chunk_left = chunk_left_.get();
     pa.split_left_total = split_left_total_.get(); pa.leaves = leaves_.get(); pa.child_init = ca.child_init; pa.hist_tasks = hist_tasks_.get(); pa.rows_per_block = rpb;
     pa.world = dp ? world_ : 1;
@@ -518,7 +518,7 @@ Tree* CudaEngine::TrainTree(int class_id, int tree_index) {
     FB_CUDA(cudaMemcpyAsync(db, hb, blob_bytes, cudaMemcpyHostToDevice, stream_));
     PartArgs pa = PartArgs();
     pa.rows = dd_->rows.get(); pa.row_stride = dd_->row_stride; pa.idx[0] = idx_[0].get(); pa.idx[1] = idx_[1].get();
-    pa.cols = dd_->cols.size() ? dd_->cols.get() : nullptr; pa.col_stride = n_;
+    pa.cols = dd_->cols.size() ? dd_->cols.get() : nullptr; pa.col_stride = dd_->col_stride();
     pa.splits = reinterpret_cast<const PartSplit*>(db); pa.num_splits = S; pa.total_chunks = chunk_cursor; pa.bits = bits_.get(); pa.chunk_left = chunk_left_.get();
     pa.split_left_total = split_left_total_.get(); pa.leaves = leaves_.get(); pa.child_init = reinterpret_cast<const ChildInit*>(db + sizeof(PartSplit) * S);
     pa.hist_tasks = hist_tasks_.get(); pa.rows_per_block = ha.rows_per_block;
