@@ -17,6 +17,7 @@ __global__ void __launch_bounds__(kCtrlThreads) LevelControllerKernel(CtrlArgs a
 // between quantization and the root histogram): the root leaf record, the level record of the root level,
 // the frontier, the root's construct task and its search descriptor.
 __global__ void InitTreeKernel(TreeInitArgs a) {
+  ChainWait();
   LeafInfo L;
   L.begin = 0; L.count = a.n_local; L.buffer = 0; L.depth = 0; L.hist_slot = 0; L.num_data_global = static_cast<int>(a.n_global);
   if (a.quant) {
@@ -42,7 +43,7 @@ __global__ void InitTreeKernel(TreeInitArgs a) {
 }  // namespace
 
 void LaunchInitTree(const TreeInitArgs& a, cudaStream_t s) {
-  InitTreeKernel<<<1, 1, 0, s>>>(a);
+  LaunchChained(true, InitTreeKernel, dim3(1), dim3(1), 0, s, a);
   FB_LAUNCHED(); FB_KERNEL_CHECK();
 }
 

@@ -32,6 +32,25 @@ inline std::atomic<int64_t>& LaunchCounter() { static std::atomic<int64_t> c{0};
 inline bool DebugSyncLaunches() { static const bool v = getenv("FALCATA_DEBUG_SYNC") != nullptr || DebugFlags::Get().sync; return v; }
 #define FB_KERNEL_CHECK() do { FB_CUDA(cudaGetLastError()); if (::fb::DebugSyncLaunches()) FB_CUDA(cudaDeviceSynchronize()); } while (0)
 
+// Chained launches: the kernels of a round run one behind the other in one stream and each is a few microseconds long, so the
+// gap between the end of one and the start of the next counts. A kernel launched with LaunchChained may be set up (its blocks
+// resident, waiting) while its predecessor drains; ChainWait - the FIRST statement of such a kernel, in every block - returns
+// once the predecessor has finished and its writes are visible, and lets the kernel's own successor be set up.
+// Measured on B200: 100 rounds of 31 leaves on 10k rows (24 launches a tree) 48.5 -> 44 ms.
+__device__ __forceinline__ void ChainWait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+// `chained` false: an ordinary launch (ChainWait then returns at once).
+template <typename... P, typename... A>
+inline void LaunchChained(bool chained, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization; attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = s; cfg.attrs = attr; cfg.numAttrs = chained ? 1 : 0;
+  FB_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
+}
+
 template <typename T>
 class DevBuf {
  public:

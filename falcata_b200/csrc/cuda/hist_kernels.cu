@@ -327,6 +327,7 @@ constexpr int kLaneMaxThreads = 1024;
 // MODE 0: integer; 1: fp32 load-add-store (pairs, a tile per warp, at most 16 warps); 2: fp32 reduction adds (planes).
 template <int NB, int kLaneStages, int MODE>
 __global__ void __launch_bounds__(MODE == 1 ? kLaneMaxThreads / 2 : kLaneMaxThreads, 1) HistQuantLaneKernel(HistArgs a) {
+  ChainWait();
   constexpr bool FLT = MODE != 0;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr int kTile = NB * 32 * (FLT ? 2 : 1);   // 4-byte cells of a tile
@@ -667,7 +668,7 @@ static void LaunchLane(const HistArgs& a, cudaStream_t s, const LaneGeometry& g)
   {                                                                                                                                \
     static bool attr = false;                                                                                                      \
     if (!attr) { FB_CUDA(cudaFuncSetAttribute(HistQuantLaneKernel<NB, ST, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024)); attr = true; } \
-    HistQuantLaneKernel<NB, ST, MODE><<<grid, g.warps * 32, g.smem, s>>>(b);                                                       \
+    LaunchChained(b.sig.world <= 1, HistQuantLaneKernel<NB, ST, MODE>, grid, dim3(g.warps * 32), g.smem, s, b);                     \
   }
 #define FB_LANE_ST(NB) { if (g.stages == 2) FB_LANE(NB, 2) else if (g.stages == 3) FB_LANE(NB, 3) else FB_LANE(NB, 4) }
   if (a.lane_bins == 16) FB_LANE_ST(16)

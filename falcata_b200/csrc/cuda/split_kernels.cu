@@ -441,6 +441,7 @@ union TailShared { ReduceShared r; CtrlShared c; };
 
 template <bool QUANT>
 __global__ void __launch_bounds__(kFindThreads, 2) FindSplitsKernel(FindArgs a, CtrlArgs ca) {
+  ChainWait();
   __shared__ int s_last;
   __shared__ CandLite s_cand[kFindThreads / 32];
   TailShared& S = *reinterpret_cast<TailShared*>(find_smem);   // used once the block's search is over
@@ -589,7 +590,7 @@ void LaunchFindSplits(const FindArgs& a, cudaStream_t s, const CtrlArgs* tail_ct
     attr = true;
   }
   const CtrlArgs ca = tail_ctrl != nullptr ? *tail_ctrl : CtrlArgs();
-  if (a.quant) FindSplitsKernel<true><<<grid, warps * 32, sm, s>>>(a, ca); else FindSplitsKernel<false><<<grid, warps * 32, sm, s>>>(a, ca);
+  LaunchChained(a.wait.world <= 1 && a.wait_best.world <= 1, a.quant ? FindSplitsKernel<true> : FindSplitsKernel<false>, grid, dim3(warps * 32), sm, s, a, ca);
   FB_LAUNCHED(); FB_KERNEL_CHECK();
 }
 
