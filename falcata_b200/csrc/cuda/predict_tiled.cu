@@ -188,38 +188,44 @@ PredictTiledKernel(const unsigned char* __restrict__ blob, const ChunkDesc* __re
 
 // Nodes of one tree in sibling-adjacent order, root first, then every split's two children next to each other, placed at
 // byte `base` of their chunk. slot_base: slot of the tile's first feature row; leaf_slot: slot of the row of -infinity.
-bool PackTree(const Tree& T, const std::vector<int>& slot_of_feature, int slot_base, int leaf_slot, bool leaf_index, int base, std::vector<PackedNode>* out,
-              std::vector<std::pair<int, int>>* queue) {
-  const int L = T.num_leaves;
-  out->resize(std::max(1, 2 * L - 1));
+void PackTree(const Tree& T, const std::vector<int>& slot_of_feature, int slot_base, int leaf_slot, bool leaf_index, int base, PackedNode* out) {
   auto offset = [&](int pos) { return static_cast<unsigned int>(base + pos * static_cast<int>(sizeof(PackedNode))); };
-  auto leaf_node = [&](int leaf, int pos) {
-    PackedNode nd;
-    if (leaf_index) std::memcpy(&nd.value, &leaf, sizeof(int)); else nd.value = static_cast<float>(T.leaf_value[leaf]);
-    nd.meta = (static_cast<unsigned int>(leaf_slot) << 16) | offset(pos) | (kLeafType << 1);
-    return nd;
+  auto place = [&](int id, int pos) {   // host ids: >= 0 split, < 0 leaf ~id
+    if (id >= 0) return;
+    if (leaf_index) { const int leaf = ~id; std::memcpy(&out[pos].value, &leaf, sizeof(int)); } else out[pos].value = static_cast<float>(T.leaf_value[~id]);
+    out[pos].meta = (static_cast<unsigned int>(leaf_slot) << 16) | offset(pos) | (kLeafType << 1);
   };
-  if (!leaf_index) for (int l = 0; l < std::max(1, L); ++l) if (std::isnan(T.leaf_value[l])) return false;   // a leaf holds its place by -infinity <= value
-  if (L <= 1) { (*out)[0] = leaf_node(0, 0); return true; }
-  // queue of (host node id, packed position); host ids: >= 0 split, < 0 leaf ~id
-  queue->clear();
-  queue->emplace_back(0, 0);
+  if (T.num_leaves <= 1) { place(~0, 0); return; }
+  // splits in breadth-first order: (host id, packed position)
+  std::vector<std::pair<int, int>> queue; queue.reserve(T.num_leaves - 1);
+  queue.emplace_back(0, 0);
   int next_free = 1;
-  for (size_t qi = 0; qi < queue->size(); ++qi) {
-    const int id = (*queue)[qi].first, pos = (*queue)[qi].second;
-    if (id < 0) { (*out)[pos] = leaf_node(~id, pos); continue; }
-    if (T.decision_type[id] & kCategoricalMask) return false;
+  for (size_t qi = 0; qi < queue.size(); ++qi) {
+    const int id = queue[qi].first, left_pos = next_free;
+    next_free += 2;
     float thr = static_cast<float>(T.threshold[id]);
     // keep "v <= threshold" exact for float inputs: round the double threshold DOWN to float
     if (static_cast<double>(thr) > T.threshold[id]) thr = std::nextafterf(thr, -std::numeric_limits<float>::infinity());
-    const int left_pos = next_free; next_free += 2;
-    PackedNode nd;
+    PackedNode& nd = out[queue[qi].second];
     nd.value = thr;
     nd.meta = (static_cast<unsigned int>(slot_base + slot_of_feature[T.split_feature[id]]) << 16) | offset(left_pos) |
               (static_cast<unsigned int>(Tree::MissingTypeOf(T.decision_type[id])) << 1) | ((T.decision_type[id] & kDefaultLeftMask) ? 1u : 0u);
-    (*out)[pos] = nd;
-    queue->emplace_back(T.left_child[id], left_pos);
-    queue->emplace_back(T.right_child[id], left_pos + 1);
+    const int child[2] = {T.left_child[id], T.right_child[id]};
+    for (int c = 0; c < 2; ++c) { if (child[c] >= 0) queue.emplace_back(child[c], left_pos + c); else place(child[c], left_pos + c); }
+  }
+}
+
+// What the packed form asks of a tree, and what the tree brings: the features it reads and whether it has missing-aware nodes.
+bool ScanTree(const Tree& T, bool leaf_index, std::vector<char>* uses, bool* plain) {
+  if (T.is_linear || T.num_leaves > 4096) return false;
+  if ((std::max(1, 2 * T.num_leaves - 1)) * sizeof(PackedNode) + 32 > static_cast<size_t>(kTreeBytes)) return false;   // larger than a buffer
+  if (!leaf_index) for (int l = 0; l < std::max(1, T.num_leaves); ++l) if (std::isnan(T.leaf_value[l])) return false;    // a leaf holds its place by -infinity <= value
+  for (int s = 0; s < T.num_leaves - 1; ++s) {
+    if (T.decision_type[s] & kCategoricalMask) return false;
+    if (Tree::MissingTypeOf(T.decision_type[s]) != 0) *plain = false;
+    const int f = T.split_feature[s];
+    if (f < 0 || f >= static_cast<int>(uses->size())) return false;
+    (*uses)[f] = 1;
   }
   return true;
 }
@@ -232,22 +238,26 @@ bool DevicePredictTiled(const GBDT* gbdt, const void* device_data, int dtype, in
                         bool leaf_index, float inv_avg, float* out_device, cudaStream_t s) {
   if (num_trees <= 0 || nrow <= 0) return false;
   if (dtype != kF32 && dtype != kF64 && dtype != kF16) return false;
+  // Packing is host work of every call (a quarter million nodes took 1.8 ms on one core): large forests are scanned and packed
+  // by all cores, straight into the one buffer that goes to the device in one copy.
+  long long forest_nodes = 0;
+  for (int t = first_tree; t < first_tree + num_trees; ++t) forest_nodes += 2LL * gbdt->models_[t]->num_leaves - 1;
+  const bool parallel = forest_nodes > (1 << 15);
   // features the forest reads, in ascending order
-  std::vector<int> slot_of_feature(std::max(1, gbdt->max_feature_idx_ + 1), -1);
-  bool plain = true;   // no node with a missing type: NaN reads as 0 everywhere, zero is an ordinary value
-  for (int t = first_tree; t < first_tree + num_trees; ++t) {
-    const Tree& T = *gbdt->models_[t];
-    if (T.is_linear) return false;
-    for (int sidx = 0; sidx < T.num_leaves - 1; ++sidx) {
-      if (T.decision_type[sidx] & kCategoricalMask) return false;
-      if (Tree::MissingTypeOf(T.decision_type[sidx]) != 0) plain = false;
-      const int f = T.split_feature[sidx];
-      if (f < 0 || f >= static_cast<int>(slot_of_feature.size())) return false;
-      slot_of_feature[f] = 0;
-    }
+  const size_t nfeat = std::max(1, gbdt->max_feature_idx_ + 1);
+  std::vector<char> uses(nfeat, 0);
+  bool plain = true, covered = true;   // plain: no node with a missing type - NaN reads as 0 everywhere, zero is an ordinary value
+#pragma omp parallel num_threads(parallel ? TeamThreads() : 1)
+  {
+    std::vector<char> mine(nfeat, 0); bool my_plain = true, my_covered = true;
+#pragma omp for schedule(static) nowait
+    for (int t = 0; t < num_trees; ++t) my_covered = my_covered && ScanTree(*gbdt->models_[first_tree + t], leaf_index, &mine, &my_plain);
+#pragma omp critical(fb_predict_scan)
+    { for (size_t f = 0; f < nfeat; ++f) uses[f] |= mine[f]; plain = plain && my_plain; covered = covered && my_covered; }
   }
-  std::vector<int> used;
-  for (size_t f = 0; f < slot_of_feature.size(); ++f) if (slot_of_feature[f] == 0) { slot_of_feature[f] = static_cast<int>(used.size()); used.push_back(static_cast<int>(f)); }
+  if (!covered) return false;
+  std::vector<int> slot_of_feature(nfeat, -1), used;
+  for (size_t f = 0; f < nfeat; ++f) if (uses[f]) { slot_of_feature[f] = static_cast<int>(used.size()); used.push_back(static_cast<int>(f)); }
   if (used.empty()) used.push_back(0);
   const int nu = static_cast<int>(used.size());
   // leaf indices have no general kernel to fall back to: the widest forest is the one of a 256-row tile beside two chunks
@@ -264,38 +274,45 @@ bool DevicePredictTiled(const GBDT* gbdt, const void* device_data, int dtype, in
   const int slot_base = (2 * chunk_bytes) >> (log_rows + 2);   // the tile's rows start behind the ring
   if (slot_base + nu > 0xFFFF) return false;
   // chunks: trees of one class in iteration order, as many as fit a ring buffer; the root words behind the nodes
-  std::vector<unsigned char> blob; std::vector<ChunkDesc> chunks;
-  std::vector<PackedNode> packed, nodes; std::vector<std::pair<int, int>> queue; std::vector<int> roots;
+  struct Place { int chunk, base, pos; };   // pos: the tree's number in its chunk
+  std::vector<Place> place(num_trees);
+  std::vector<ChunkDesc> chunks;
+  size_t bytes = 0;
   for (int cls = 0; cls < K; ++cls) {
-    int first = -1;
+    ChunkDesc d; d.ntrees = 0; d.roots = 0; d.cls = cls; d.first_tree = 0; d.pad = 0;
     auto close = [&]() {
-      if (roots.empty()) return;
-      ChunkDesc d; d.offset = static_cast<long long>(blob.size()); d.ntrees = static_cast<int>(roots.size()); d.cls = cls; d.first_tree = first; d.pad = 0;
-      d.roots = static_cast<int>(nodes.size() * sizeof(PackedNode));
-      const size_t bytes = (d.roots + roots.size() * 4 + 15) & ~static_cast<size_t>(15);
-      d.bytes = static_cast<int>(bytes);
-      blob.resize(blob.size() + bytes, 0);
-      memcpy(blob.data() + d.offset, nodes.data(), nodes.size() * sizeof(PackedNode));
-      memcpy(blob.data() + d.offset + d.roots, roots.data(), roots.size() * 4);
-      chunks.push_back(d); roots.clear(); nodes.clear(); first = -1;
+      if (d.ntrees == 0) return;
+      d.offset = static_cast<long long>(bytes); d.bytes = (d.roots + d.ntrees * 4 + 15) & ~15;
+      bytes += d.bytes;
+      chunks.push_back(d); d.ntrees = 0; d.roots = 0;
     };
     for (int t = cls; t < num_trees; t += K) {
-      const Tree& T = *gbdt->models_[first_tree + t];
-      const size_t tree_nodes = std::max(1, 2 * T.num_leaves - 1);
-      if (T.num_leaves > 4096 || tree_nodes * sizeof(PackedNode) + 32 > static_cast<size_t>(kTreeBytes)) return false;   // a single tree larger than a buffer
-      const size_t need = (nodes.size() + tree_nodes) * sizeof(PackedNode) + (roots.size() + 1) * 4 + 16;
-      if (need > static_cast<size_t>(chunk_bytes)) close();
-      const int base = static_cast<int>(nodes.size() * sizeof(PackedNode));
-      if (!PackTree(T, slot_of_feature, slot_base, slot_base + nu, leaf_index, base, &packed, &queue)) return false;
-      if (first < 0) first = t;
-      roots.push_back(base);
-      nodes.insert(nodes.end(), packed.begin(), packed.end());
+      const int tree = std::max(1, 2 * gbdt->models_[first_tree + t]->num_leaves - 1) * static_cast<int>(sizeof(PackedNode));
+      if (d.roots + tree + (d.ntrees + 1) * 4 + 16 > chunk_bytes) close();
+      if (d.ntrees == 0) d.first_tree = t;
+      place[t] = {static_cast<int>(chunks.size()), d.roots, d.ntrees};
+      d.roots += tree; ++d.ntrees;
     }
     close();
   }
   if (chunks.empty()) return false;
-  DevBuf<unsigned char> d_blob; DevBuf<ChunkDesc> d_chunks; DevBuf<int> d_used;
-  d_blob.Upload(blob, s); d_chunks.Upload(chunks, s); d_used.Upload(used, s);
+  // one buffer, one copy: chunk list, used features, trees
+  const size_t chunks_at = 0, used_at = chunks.size() * sizeof(ChunkDesc), blob_at = (used_at + used.size() * sizeof(int) + 15) & ~static_cast<size_t>(15);
+  std::vector<unsigned char> staged(blob_at + bytes);
+  memcpy(staged.data() + chunks_at, chunks.data(), chunks.size() * sizeof(ChunkDesc));
+  memcpy(staged.data() + used_at, used.data(), used.size() * sizeof(int));
+#pragma omp parallel for schedule(static) num_threads(parallel ? TeamThreads() : 1)
+  for (int t = 0; t < num_trees; ++t) {
+    const ChunkDesc& d = chunks[place[t].chunk];
+    unsigned char* chunk = staged.data() + blob_at + d.offset;
+    PackTree(*gbdt->models_[first_tree + t], slot_of_feature, slot_base, slot_base + nu, leaf_index, place[t].base, reinterpret_cast<PackedNode*>(chunk + place[t].base));
+    reinterpret_cast<int*>(chunk + d.roots)[place[t].pos] = place[t].base;
+  }
+  DevBuf<unsigned char> forest;
+  forest.Upload(staged.data(), staged.size(), s);
+  const unsigned char* d_blob = forest.get() + blob_at;
+  const ChunkDesc* d_chunks = reinterpret_cast<const ChunkDesc*>(forest.get() + chunks_at);
+  const int* d_used = reinterpret_cast<const int*>(forest.get() + used_at);
   const int tiles = (nrow + (1 << log_rows) - 1) >> log_rows;
   const int grid = std::min(tiles, sms);
   const int nc = static_cast<int>(chunks.size());
@@ -303,7 +320,7 @@ bool DevicePredictTiled(const GBDT* gbdt, const void* device_data, int dtype, in
   {                                                                                                                                \
     static bool attr = false;                                                                                                      \
     if (!attr) { FB_CUDA(cudaFuncSetAttribute(PredictTiledKernel<T, LEAF, PLAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPredictSmem)); attr = true; } \
-    PredictTiledKernel<T, LEAF, PLAIN><<<grid, kPredictThreads, smem, s>>>(d_blob.get(), d_chunks.get(), nc, chunk_bytes, d_used.get(), nu, static_cast<const T*>(device_data), nrow, ncol, \
+    PredictTiledKernel<T, LEAF, PLAIN><<<grid, kPredictThreads, smem, s>>>(d_blob, d_chunks, nc, chunk_bytes, d_used, nu, static_cast<const T*>(device_data), nrow, ncol, \
                                                                            row_major ? 1 : 0, log_rows, K, num_trees, inv_avg, out_device);   \
   }
 #define FB_TILED(T, LEAF) { if (plain) FB_TILED_P(T, LEAF, true) else FB_TILED_P(T, LEAF, false) }
