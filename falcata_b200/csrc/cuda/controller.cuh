@@ -28,13 +28,18 @@ struct CtrlShared {
   int ncand, nkeep, total_chunks, total_blocks;
 };
 
-// A record that another block of the SAME launch may have written a moment ago: read through L2, in 8-byte pieces
+// A record that another block of the SAME launch may have written a moment ago: read through L2, in 16- or 8-byte pieces
 // where the type allows it (the loads of one record are independent and issue back to back).
 template <typename T>
 __device__ inline T LoadWords(const T* p) {
   static_assert(sizeof(T) % 4 == 0, "word-sized records only");
   T v;
-  if constexpr (sizeof(T) % 8 == 0 && alignof(T) >= 8) {
+  if constexpr (sizeof(T) % 16 == 0 && alignof(T) >= 16) {
+    const uint4* s = reinterpret_cast<const uint4*>(p);
+    uint4* d = reinterpret_cast<uint4*>(&v);
+#pragma unroll
+    for (int w = 0; w < static_cast<int>(sizeof(T) / 16); ++w) d[w] = __ldcg(s + w);
+  } else if constexpr (sizeof(T) % 8 == 0 && alignof(T) >= 8) {
     const unsigned long long* s = reinterpret_cast<const unsigned long long*>(p);
     unsigned long long* d = reinterpret_cast<unsigned long long*>(&v);
 #pragma unroll

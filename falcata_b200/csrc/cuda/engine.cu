@@ -411,11 +411,11 @@ int CudaEngine::ChooseRowsPerBlock(long long total_rows) const {
     long long rpb = (total_rows / (4LL * num_sms_) + unit - 1) / unit * unit;
     if (!quant_) {
       // fp32: every block clears and merges whole tiles of float pairs and nothing can overflow, so fewer, longer blocks:
-      // about two waves over all 32-group parts, no shorter than two stages of all warps
+      // about two waves over all 32-group parts, no shorter than one stage of all warps
       const long long parts = (train_->num_groups + 31) / 32;
       const long long row_blocks = std::max<long long>(1, 2LL * num_sms_ / parts);
       rpb = (total_rows / row_blocks + unit - 1) / unit * unit;
-      return static_cast<int>(std::max<long long>(rpb, 2LL * unit));
+      return static_cast<int>(std::max<long long>(rpb, unit));
     }
     rpb = std::min<long long>(std::max<long long>(rpb, 3LL * unit), 13LL * unit);
     rpb = std::min<long long>(rpb, static_cast<long long>(LaneTiles(lane_red_, sub_rows_, lane_bins_, !quant_)) * (sub_rows_ / 32 * 32));

@@ -208,7 +208,7 @@ Tree* CudaEngine::TrainTree(int class_id, int tree_index) {
   const bool dp = data_parallel();
   const bool rs = dp && !voting_;   // construct fused with the reduce-scatter (plain data-parallel)
   ha.dest.bin_owner = bin_owner_.get(); ha.dest.bin_local = voting_ ? bin_identity_.get() : bin_local_.get(); ha.dest.num_ranks = rs ? world_ : 1; ha.dest.rank = rank_;
-  ha.dest.owner_only = feature_parallel_ ? 1 : 0;
+  ha.dest.owner_only = feature_parallel_ ? 1 : 0; ha.dest.identity = world_ <= 1 || voting_ ? 1 : 0;
   for (int r = 0; r < kMaxRanks; ++r) { ha.dest.pool[r] = nullptr; ha.dest.slot_stride[r] = 0; }
   for (int r = 0; r < kMaxRanks; ++r) ha.dest.peer_stage[r] = nullptr;
   if (rs) {

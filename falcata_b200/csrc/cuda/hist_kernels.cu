@@ -91,29 +91,29 @@ __device__ inline bool PushTaskIfLast(const HistArgs& a, int ti, const HistTask&
 // Measured (mean launch of a tree): 1M x 100 groups of 255 bins, fp32, 156 -> 116 us; 515k x 90, integer, 65 -> 43 us.
 // A task with a single block stores (its cells were cleared with the pool; nobody else adds to them). All threads of the block
 // call Write between two rounds of Put.
+// (start, count): the groups' places in the bin space, in shared memory since the block's start - the tiles leave the SM a few
+// KB of L1, and every look-up of the flush would go to L2.
 template <bool FLT, int NB>
 struct BlockFlush {
   static constexpr int kBins = NB < 128 ? NB : 128, kPitch = kBins + 1, kBytes = 32 * kPitch * (FLT ? 16 : 8);
-  const HistArgs& a; int group0; bool single; unsigned char* stage; char* base; bool identity;
-  __device__ BlockFlush(const HistArgs& args, const HistTask& task, int ti, int first_group, bool single_block, unsigned char* scratch)
-      : a(args), group0(first_group), single(single_block), stage(scratch) {
+  const HistArgs& a; const int* start; const int* count; int ngroups; bool single; unsigned char* stage; char* base; bool identity;
+  __device__ BlockFlush(const HistArgs& args, const HistTask& task, int ti, const int* group_start, const int* group_count, int groups, bool single_block, unsigned char* scratch)
+      : a(args), start(group_start), count(group_count), ngroups(groups), single(single_block), stage(scratch) {
     const HistDest& d = a.dest;
-    identity = d.num_ranks > 1;   // the staging histogram of a task holds the bins in their global order
-    const long long cell = identity ? static_cast<long long>(ti) * a.num_total_bin : static_cast<long long>(task.slot) * d.slot_stride[0];
-    base = static_cast<char*>(identity ? d.stage_local : d.pool[0]) + cell * (FLT ? 16 : 8);
+    const bool staged = d.num_ranks > 1;   // the staging histogram of a task holds the bins in their global order
+    const long long cell = staged ? static_cast<long long>(ti) * a.num_total_bin : static_cast<long long>(task.slot) * d.slot_stride[0];
+    base = static_cast<char*>(staged ? d.stage_local : d.pool[0]) + cell * (FLT ? 16 : 8);
+    identity = staged || d.identity != 0;
   }
   __device__ void Put(int group, int bin, int word, double v) { reinterpret_cast<double*>(stage)[(group * kPitch + bin) * 2 + word] = v; }
   __device__ void Put(int group, int bin, hist_q_t v) { reinterpret_cast<hist_q_t*>(stage)[group * kPitch + bin] = v; }
   __device__ void Write(int bin0) {
     __syncthreads();
     constexpr int kWords = FLT ? 2 : 1, row = kBins * kWords;
-    const int ngroups = min(32, a.num_groups - group0);
     for (int e = threadIdx.x; e < ngroups * row; e += blockDim.x) {
       const int g = e / row, k = e % row, b = bin0 + k / kWords;
-      const int start = a.group_bin_start[group0 + g];
-      const int count = a.group_bin_count != nullptr ? a.group_bin_count[group0 + g] : (group0 + g + 1 < a.num_groups ? a.group_bin_start[group0 + g + 1] : a.num_total_bin) - start;
-      if (b >= count) continue;
-      const int local = identity ? start + b : a.dest.bin_local[start + b];
+      if (b >= count[g]) continue;
+      const int bin = start[g] + b, local = identity ? bin : a.dest.bin_local[bin];
       if constexpr (FLT) {
         const double v = reinterpret_cast<const double*>(stage)[g * 2 * kPitch + k];
         if (v == 0.0) continue;
@@ -121,7 +121,7 @@ struct BlockFlush {
         if (single) *p = v; else atomicAdd(p, v);
       } else {
         const hist_q_t v = reinterpret_cast<const hist_q_t*>(stage)[g * kPitch + k];
-        if (v == 0 || (a.dest.owner_only && a.dest.bin_owner[start + b] != a.dest.rank)) continue;
+        if (v == 0 || (a.dest.owner_only && a.dest.bin_owner[bin] != a.dest.rank)) continue;
         hist_q_t* p = reinterpret_cast<hist_q_t*>(base) + local;
         if (single) *p = v; else atomicAdd(p, v);
       }
@@ -351,6 +351,12 @@ __global__ void __launch_bounds__(MODE == 1 ? kLaneMaxThreads / 2 : kLaneMaxThre
   const int nrows = static_cast<int>(max(0LL, min(static_cast<long long>(a.rows_per_block), task.count - row0)));
   const int g0 = blockIdx.y * 32;
   const int ng = min(32, a.num_groups - g0);
+  __shared__ int s_gstart[32], s_gcount[32];   // for the flush; read after a block barrier
+  if (threadIdx.x < ng) {
+    const int g = g0 + threadIdx.x, start = a.group_bin_start[g];
+    s_gstart[threadIdx.x] = start;
+    s_gcount[threadIdx.x] = a.group_bin_count != nullptr ? a.group_bin_count[g] : (g + 1 < a.num_groups ? a.group_bin_start[g + 1] : a.num_total_bin) - start;
+  }
   const int byte0 = a.pack4 ? g0 / 2 : g0;                       // first byte of this 32-group part inside the row
   const int copy16 = a.pack4 ? 1 : min(2, (a.row_stride - g0) / 16);   // 16-byte pieces of this part inside the row
   int* tile = tiles + (warp / share) * kTile;
@@ -463,7 +469,7 @@ __global__ void __launch_bounds__(MODE == 1 ? kLaneMaxThreads / 2 : kLaneMaxThre
   __syncthreads();
   // the tiles of a block are summed in tile order (fp32: in double)
   using Flush = BlockFlush<FLT, NB>;
-  Flush flush(a, task, ti, g0, row_blocks == 1, smem_raw + sizeof(int) * ntiles * kTile);
+  Flush flush(a, task, ti, s_gstart, s_gcount, ng, row_blocks == 1, smem_raw + sizeof(int) * ntiles * kTile);
   for (int b0 = 0; b0 < NB; b0 += Flush::kBins) {
     for (int b = warp; b < Flush::kBins; b += kLaneWarps) {
       const int cell = (b0 + b) * 32 + lane;

@@ -13,7 +13,7 @@ namespace fb {
 // Device-resident state of the level loop. With the device controller the host enqueues the kernels
 // of several levels ahead with upper-bound grids; every kernel reads how much work the level really
 // has from this record, which the controller kernel rewrites between levels.
-struct LevelCtrl {
+struct alignas(16) LevelCtrl {
   int num_leaves, next_slot, done, level;
   int num_splits, num_children, total_chunks, total_blocks;
   int frontier_count, journal_count, pad0;
@@ -21,7 +21,7 @@ struct LevelCtrl {
   int skip_search;   // 1: this level used up the leaf budget - its children can never split, so their construct and search are skipped
 };
 // One applied split, in application order: enough for the host to rebuild the tree after the last level.
-struct SplitJournal { int leaf, right_leaf, parent_global, pad; int begin, count, buffer, depth; /* the parent's window and depth */ SplitRecord rec; };
+struct alignas(16) SplitJournal { int leaf, right_leaf, parent_global, pad; int begin, count, buffer, depth; /* the parent's window and depth */ SplitRecord rec; };
 struct ChildInit;
 
 // ------------------------------------------------------------- objective ----
@@ -57,6 +57,7 @@ struct HistDest {
   const unsigned char* bin_owner;  // [num_total_bin]
   const int* bin_local;            // [num_total_bin]
   int num_ranks, rank;
+  int identity;                    // 1: bin_local is the identity (every rank's pool but that of a feature-parallel or reduce-scattered run)
   int owner_only;                  // feature-parallel: every rank sees all rows; only bins of owned features are kept (no exchange)
   // num_ranks > 1: blocks add into a LOCAL staging histogram of their task; the last block of a
   // task to finish stores the finished slices into the owner ranks' per-source staging slots
@@ -106,9 +107,9 @@ bool LaunchHistConstructQuantTC(const HistArgs& a, cudaStream_t s);
 int HistTcRowsPerBlock(long long count, int num_sms);
 
 // ------------------------------------------------------------ split find ----
-struct FindChild { int leaf; int slot; int other_slot; int is_larger; int split; int is_left; int parent_global; int task; };   // task: construct task of this pair's smaller child   // larger: bins = pool[slot] - pool[other_slot], written back to pool[slot]
+struct alignas(16) FindChild { int leaf; int slot; int other_slot; int is_larger; int split; int is_left; int parent_global; int task; };   // task: construct task of this pair's smaller child   // larger: bins = pool[slot] - pool[other_slot], written back to pool[slot]
 
-struct CandLite {      // best threshold of one (child, feature)
+struct alignas(16) CandLite {      // best threshold of one (child, feature)
   double gain; int feature; int threshold; int default_left; int left_cnt;
   long long left_gi, left_hi; double left_g, left_h;
   int is_categorical, num_cat_bins; uint32_t cat_bitset[8];   // categorical: the bins that go left
@@ -234,7 +235,7 @@ void LaunchGatherBest(const FindArgs& a, cudaStream_t s);      // world > 1: arg
 
 // ------------------------------------------------------------- partition ----
 constexpr int kPartChunk = 2048;
-struct ChildInit {     // host-decided child bookkeeping of one split
+struct alignas(16) ChildInit {     // host-decided child bookkeeping of one split
   int left_slot, right_slot;       // histogram slots of the children
   int smaller_is_left;
   double left_g, left_h, right_g, right_h, left_out, right_out;

@@ -82,7 +82,7 @@ int FB_OpHistogram(const uint8_t* rows, int row_stride, int num_groups, const vo
     d_task.Upload(&t, 1, s);
   }
   for (int r = 0; r < 8; ++r) { a.dest.pool[r] = nullptr; a.dest.slot_stride[r] = 0; }
-  a.dest.pool[0] = pool.get(); a.dest.slot_stride[0] = total; a.dest.bin_owner = d_owner.get(); a.dest.bin_local = d_local.get(); a.dest.num_ranks = 1; a.dest.rank = 0;
+  a.dest.pool[0] = pool.get(); a.dest.slot_stride[0] = total; a.dest.bin_owner = d_owner.get(); a.dest.bin_local = d_local.get(); a.dest.num_ranks = 1; a.dest.rank = 0; a.dest.identity = 1;
   if (quant) LaunchHistConstructQuant(a, s); else LaunchHistConstructFloat(a, s);
   FB_CUDA(cudaStreamSynchronize(s));
   if (quant) {

@@ -440,7 +440,7 @@ __device__ inline void GatherChild(const FindArgs& a, int child) {
 union TailShared { ReduceShared r; CtrlShared c; };
 
 template <bool QUANT>
-__global__ void __launch_bounds__(kFindThreads, 2) FindSplitsKernel(FindArgs a, CtrlArgs ca) {
+__global__ void __launch_bounds__(kFindThreads) FindSplitsKernel(FindArgs a, CtrlArgs ca) {
   ChainWait();
   __shared__ int s_last;
   __shared__ CandLite s_cand[kFindThreads / 32];

@@ -36,7 +36,7 @@ struct Metadata {
 };
 
 // What split finding needs to know about one inner feature.
-struct FeatureMeta {
+struct alignas(16) FeatureMeta {   // (16-byte pieces: the device kernels load and store whole records)
   int hist_offset;     // first histogram slot of this feature's bins (group start + offset in group)
   int num_bin;         // bins of the feature itself
   int missing_type;    // MissingType

@@ -41,7 +41,7 @@ struct SplitParams {
 
 // Fixed-size record of the best split of one leaf (or one (leaf, feature) task). POD: it is
 // written by device kernels, copied between ranks and read by the host.
-struct SplitRecord {
+struct alignas(16) SplitRecord {   // (16-byte pieces: the device kernels load and store whole records)
   double gain;            // gain above the leaf's own (already minus min_gain_shift); <= 0 / -inf: none
   int feature;            // inner feature index, -1 when no split
   int threshold;          // bin index: feature bin <= threshold goes left (numerical)
