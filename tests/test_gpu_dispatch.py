@@ -1,0 +1,124 @@
+"""Kernel variants that a rule on sizes selects, at the edges of the rule: the lane construct's block flush, the one-launch row
+partition, the split search, the per-row kernels of a round's set-up and the tile shapes of prediction."""
+import numpy as np
+import pytest
+import torch
+
+import falcata_b200 as fb
+from util import make_binary, model_body
+
+pytestmark = pytest.mark.gpu
+
+
+def _rows(n, groups, nb, gen):
+    stride = ((groups + 4 + 15) // 16) * 16
+    rows = torch.full((n, stride), 255, dtype=torch.uint8, device="cuda")   # bytes past the last group are no bins
+    rows[:, :groups] = torch.randint(0, nb, (n, groups), generator=gen, device="cuda", dtype=torch.int32).to(torch.uint8)
+    rows[: n // 2, 0] = nb - 1   # runs of one bin: equal cells inside a step are forwarded in registers
+    return rows
+
+
+def _reference(rows, groups, nb, value, idx=None):
+    sel = rows if idx is None else rows[idx.long()]
+    v = (value if idx is None else value[idx.long()]).double()
+    out = torch.zeros(groups * nb, dtype=torch.float64, device="cuda")
+    for k in range(groups):
+        out.index_add_(0, sel[:, k].long() + k * nb, v)
+    return out
+
+
+@pytest.mark.parametrize("nb", [16, 17, 64, 65, 128, 129, 256])
+@pytest.mark.parametrize("n,groups,rpb", [(1, 1, 512), (31, 16, 512), (33, 17, 64), (2049, 28, 512), (20011, 32, 4096), (9001, 33, 1024), (5003, 49, 96)])
+def test_lane_construct(n, groups, nb, rpb):
+    from falcata_b200 import ops
+    gen = torch.Generator(device="cuda"); gen.manual_seed(n * 1000 + groups + nb)
+    rows = _rows(n, groups, nb, gen)
+    idx = torch.randperm(n, generator=gen, device="cuda")[: max(1, (2 * n) // 3)].int()
+    for qbins in (4, 64):
+        gi = torch.randint(-(qbins // 2), qbins // 2 + 1, (n,), generator=gen, device="cuda", dtype=torch.int32)
+        hi = torch.randint(0, qbins + 1, (n,), generator=gen, device="cuda", dtype=torch.int32)
+        packed = (gi << 16) | (hi & 0xFFFF)
+        for mode in (1, 2):
+            for sub in (None, idx):
+                out = ops.histogram(rows, packed, [nb] * groups, idx=sub, quant=True, quant_bins=qbins, rows_per_block=rpb, lane_mode=mode)
+                assert torch.equal(out[:, 0], _reference(rows, groups, nb, gi, sub).long()) and torch.equal(out[:, 1], _reference(rows, groups, nb, hi, sub).long())
+    gh = torch.randn(n, 2, device="cuda", generator=gen); gh[:, 1].abs_()
+    for mode in (1, 2):   # load-add-store, reduction adds
+        for sub in (None, idx):
+            out = ops.histogram(rows, gh, [nb] * groups, idx=sub, quant=False, rows_per_block=rpb, lane_mode=mode)
+            count = _reference(rows, groups, nb, torch.ones(n, device="cuda"), sub)
+            for k in range(2):
+                # fp32 sums of a cell's rows: at most `count` roundings of a running sum of at most sum |v|
+                bound = count * 2.0 ** -24 * _reference(rows, groups, nb, gh[:, k].abs(), sub) + 1e-12
+                assert bool(((out[:, k] - _reference(rows, groups, nb, gh[:, k], sub)).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("n", [1, 3, 4, 5, 1023, 148 * 8 * 256 * 4 + 3])
+def test_quantize_walks_every_row(n):
+    from falcata_b200 import ops
+    g = torch.randn(n, device="cuda"); h = torch.rand(n, device="cuda")
+    packed, scales, sums = ops.quantize(g, h, 64, False, seed=7, iter_key=3)
+    assert torch.equal(scales, torch.stack([g.abs().max() / 32, h.max() / 64]))
+    assert torch.equal(sums, torch.stack([(packed >> 16).long().sum(), (packed & 0xFFFF).long().sum()]))
+    # rounding to the nearest level: half a level, and one unit in the last place of a product of at most 64
+    assert float(((packed >> 16) * scales[0] - g).abs().max()) <= float(scales[0]) * (0.5 + 1e-5)
+    # the same words from buffers that allow no 16-byte access
+    if n > 4:
+        g1 = torch.empty(n + 1, device="cuda")[1:]; g1.copy_(g); h1 = torch.empty(n + 1, device="cuda")[1:]; h1.copy_(h)
+        assert torch.equal(ops.quantize(g1, h1, 64, False, seed=7, iter_key=3)[0], packed)
+
+
+@pytest.mark.parametrize("extra", [{}, {"bagging_fraction": 0.7, "bagging_freq": 1}, {"grow_policy": "leaf"}, {"use_missing": True, "nan": 0.2}])
+@pytest.mark.parametrize("n", [2047, 2049, 150001])
+def test_one_launch_partition_gives_the_same_model(n, extra):
+    """More chunks of a split than one look-back window (32 x 2048 rows), a window that is one chunk, and one row more."""
+    X, y = make_binary(n, 12)
+    extra = dict(extra)
+    X[np.random.RandomState(0).rand(*X.shape) < extra.pop("nan", 0.0)] = np.nan
+    p = dict({"objective": "binary", "num_leaves": 63, "max_bin": 63, "verbosity": -1, "quant_mode": "stochastic", "quant_bins": 4, "device_type": "cuda", "min_data_in_leaf": 3}, **extra)
+    models = [model_body(fb.train(dict(p, cuda_plan=plan), fb.Dataset(X, y), 5).model_to_string()) for plan in ("auto", "auto,fused_scan:off")]
+    assert models[0] == models[1]
+
+
+@pytest.mark.parametrize("features", [1, 8, 9, 16, 17, 40])
+@pytest.mark.parametrize("max_bin", [7, 31, 32, 33, 64, 65, 127, 255])
+def test_split_search_agrees_with_the_host(features, max_bin):
+    rng = np.random.RandomState(features * 1000 + max_bin)
+    X = rng.randn(3000, features).astype(np.float32)
+    X[rng.rand(*X.shape) < 0.1] = np.nan
+    # gradients of a custom L2 objective on a coarse grid are exact, so host and device quantize alike
+    y = (np.nan_to_num(X).sum(axis=1) + rng.randn(3000) > 0).astype(np.float32)
+    p = {"objective": "none", "num_leaves": 31, "max_bin": max_bin, "verbosity": -1, "quant_mode": "fixedpoint", "quant_bins": 16, "min_data_in_leaf": 5, "grow_policy": "level"}
+
+    def fobj(preds, ds):
+        raw = preds.cpu().numpy() if isinstance(preds, torch.Tensor) else np.asarray(preds)
+        return (np.round((raw - y) * 8) / 8).astype(np.float32), np.ones_like(y)
+
+    def trained(**kw):
+        bst = fb.Booster(dict(p, **kw), fb.Dataset(X, y, params={"max_bin": max_bin}))
+        bst.update(fobj=fobj)
+        return model_body(bst.model_to_string())
+
+    device = trained(device_type="cuda")
+    assert device == trained(device_type="cuda", cuda_plan="auto,fused_tail:off")
+    assert device == trained(device_type="cpu")
+
+
+def _forest(trees, leaves, features, seed, X):
+    rng = np.random.RandomState(seed)
+    y = (X[:, 0] + rng.randn(len(X)) > 0).astype(np.float32)
+    # random labels and one feature per split from all of them: every feature is used by some tree
+    return fb.train({"objective": "binary", "num_leaves": leaves, "verbosity": -1, "min_data_in_leaf": 1, "min_sum_hessian_in_leaf": 0, "feature_fraction": 0.05 if features > 60 else 0.5,
+                     "seed": seed}, fb.Dataset(X, y), trees)
+
+
+@pytest.mark.parametrize("rows,features,trees,leaves", [(1, 5, 3, 7), (31, 40, 70, 31), (33, 152, 60, 63), (148 * 32 + 1, 152, 40, 255), (40001, 155, 40, 63), (3001, 320, 40, 127), (257, 12, 9, 1500)])
+def test_predict_tiles_match_the_host(rows, features, trees, leaves):
+    rng = np.random.RandomState(rows)
+    X = rng.randn(max(rows, 4000), features).astype(np.float32)
+    bst = _forest(trees, leaves, features, 1, X)
+    x = X[:rows]
+    # leaf values and the sums are rounded to fp32 once each: 2^-23 of the largest partial sum, far below 1e-5
+    for t in (torch.from_numpy(x).cuda(), torch.from_numpy(x.astype(np.float64)).cuda()):
+        np.testing.assert_allclose(bst.predict(t, raw_score=True).cpu().numpy().reshape(-1), np.asarray(bst.predict(x, raw_score=True)).reshape(-1), rtol=1e-5, atol=1e-5)
+    assert np.array_equal(np.asarray(bst.predict(torch.from_numpy(x).cuda(), pred_leaf=True).cpu()).reshape(rows, -1), np.asarray(bst.predict(x, pred_leaf=True)).reshape(rows, -1))
