@@ -411,7 +411,8 @@ int CudaEngine::ChooseRowsPerBlock(long long total_rows) const {
     long long rpb = (total_rows / (4LL * num_sms_) + unit - 1) / unit * unit;
     if (!quant_) {
       // fp32: every block clears and merges whole tiles of float pairs and nothing can overflow, so fewer, longer blocks:
-      // about two waves over all 32-group parts, no shorter than one stage of all warps
+      // about two waves over all 32-group parts, no shorter than one stage of all warps (against eight stages: 50k rows x 30
+      // groups of 63 bins, ten rounds 6.1 -> 5.6 ms; against two: 10k rows x 28 of 255 bins, a hundred rounds 43 -> 39 ms)
       const long long parts = (train_->num_groups + 31) / 32;
       const long long row_blocks = std::max<long long>(1, 2LL * num_sms_ / parts);
       rpb = (total_rows / row_blocks + unit - 1) / unit * unit;
