@@ -15,6 +15,7 @@ namespace {
 
 // score[row] += v for the rows of a leaf's window, walked by gridDim.y blocks. A row is in one window, so the reduction adds
 // (nothing comes back to the SM: 32 scattered sectors per instruction once instead of twice) do not depend on their order.
+// (A global reduction add flushes a subnormal sum, below 1.2e-38, to zero.)
 // Measured at 11M rows and 255 leaves: 172 us with load, add and store, 62 us.
 __device__ __forceinline__ void AddToWindow(const LeafInfo& L, float v, const int* __restrict__ idx0, const int* __restrict__ idx1, float* __restrict__ score) {
   const int* idx = (L.buffer ? idx1 : idx0) + L.begin;
