@@ -268,9 +268,9 @@ __device__ void FindSplitsWarp(const FindArgs& a, int fi, CandLite* out) {
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       const int b = b0 + 32 * k + lane;
-      if (b >= nb) continue;
+      if (b >= nb || b == mfb) continue;   // the un-stored bin's entry has one writer: lane 0, below
       bins[entry(b)] = v[k];
-      if (write_back && b != mfb) reinterpret_cast<Bin*>(child)[(mfb >= 0 && b > mfb) ? b - 1 : b] = v[k];
+      if (write_back) reinterpret_cast<Bin*>(child)[(mfb >= 0 && b > mfb) ? b - 1 : b] = v[k];
       if constexpr (QUANT) sum_q += v[k]; else { sum_d.x += v[k].x; sum_d.y += v[k].y; }
     }
   }

@@ -104,6 +104,35 @@ def test_split_search_agrees_with_the_host(features, max_bin):
     assert device == trained(device_type="cpu")
 
 
+@pytest.mark.parametrize("zero_as_missing", [False, True])
+@pytest.mark.parametrize("quant", ["fixedpoint", "none"])
+@pytest.mark.parametrize("levels", [20, 33, 66, 130, 200])
+def test_search_of_bundled_features_agrees_with_the_host(levels, quant, zero_as_missing):
+    """Exclusive sparse columns share a byte column; the bin of zero, which lies between the negative and the positive values, is
+    not stored there and the search reconstructs it: in runs of 1, 2, 4 and 8 bins per lane."""
+    rng = np.random.RandomState(levels)
+    n, columns = 6000, [levels, 24, 12, 12]
+    which = rng.randint(0, len(columns), size=n)
+    X = np.zeros((n, len(columns) + 1), dtype=np.float32)
+    for j, k in enumerate(columns):
+        rows = np.flatnonzero(which == j)
+        v = rng.randint(1, k + 1, size=len(rows)).astype(np.float32) - k // 3   # a third of the values is negative
+        X[rows, j] = np.where(v <= 0, v - 1, v)
+    X[:, -1] = rng.randn(n)
+    # gradients of a custom L2 objective on a coarse grid: sums of 6000 of them are exact in fp32, so both learners see the same sums
+    y = (np.round((X.sum(axis=1) % 7 + which + rng.randn(n)) * 8) / 8).astype(np.float32)
+    p = {"objective": "none", "num_leaves": 31, "max_bin": 255, "verbosity": -1, "quant_mode": quant, "quant_bins": 16, "min_data_in_leaf": 5, "grow_policy": "level"}
+    bodies = []
+    for device in ("cuda", "cpu"):
+        data = fb.Dataset(X, y, params={"max_bin": 255, "min_data_in_bin": 1, "zero_as_missing": zero_as_missing})
+        bst = fb.Booster(dict(p, device_type=device), data)
+        assert data.info()["num_groups"] < X.shape[1]
+        bst.update(fobj=lambda preds, ds: (-y, np.ones_like(y)))
+        bodies.append(model_body(bst.model_to_string()))
+    assert bodies[0] == bodies[1]
+    assert any(int(t) < len(columns) for line in bodies[0].splitlines() if line.startswith("split_feature=") for t in line.split("=")[1].split())
+
+
 def _forest(trees, leaves, features, seed, X):
     rng = np.random.RandomState(seed)
     y = (X[:, 0] + rng.randn(len(X)) > 0).astype(np.float32)
