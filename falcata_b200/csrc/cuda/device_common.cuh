@@ -51,6 +51,16 @@ inline void LaunchChained(bool chained, void (*kernel)(P...), dim3 grid, dim3 bl
   FB_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
 }
 
+// Lets `kernel` be launched on the current device with up to `bytes` of dynamic shared memory (the limit is set per device).
+// `done`: one per kernel.
+template <typename K>
+inline void AllowSharedMemory(K kernel, int bytes, PerDevice* done) {
+  int device = 0; FB_CUDA(cudaGetDevice(&device));
+  if (done->Done(device)) return;
+  FB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+  done->SetDone(device);
+}
+
 template <typename T>
 class DevBuf {
  public:

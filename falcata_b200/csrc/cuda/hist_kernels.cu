@@ -672,8 +672,8 @@ static void LaunchLane(const HistArgs& a, cudaStream_t s, const LaneGeometry& g)
   HistArgs b = a; b.lane_share = g.share;
 #define FB_LANE(NB, ST)                                                                                                            \
   {                                                                                                                                \
-    static bool attr = false;                                                                                                      \
-    if (!attr) { FB_CUDA(cudaFuncSetAttribute(HistQuantLaneKernel<NB, ST, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024)); attr = true; } \
+    static PerDevice allowed;                                                                                                      \
+    AllowSharedMemory(HistQuantLaneKernel<NB, ST, MODE>, 220 * 1024, &allowed);                                                    \
     LaunchChained(b.sig.world <= 1, HistQuantLaneKernel<NB, ST, MODE>, grid, dim3(g.warps * 32), g.smem, s, b);                     \
   }
 #define FB_LANE_ST(NB) { if (g.stages == 2) FB_LANE(NB, 2) else if (g.stages == 3) FB_LANE(NB, 3) else FB_LANE(NB, 4) }
@@ -700,10 +700,10 @@ void LaunchHistConstructQuant(const HistArgs& a, cudaStream_t s) {
   (void)max_groups;
   dim3 grid(a.total_blocks, a.num_parts);
   if (two_phase) {
-    static bool attr = false; if (!attr) { FB_CUDA(cudaFuncSetAttribute(HistQuantKernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024)); attr = true; }
+    static PerDevice allowed; AllowSharedMemory(HistQuantKernel<true>, 200 * 1024, &allowed);
     HistQuantKernel<true><<<grid, kHistThreads, sm, s>>>(a);
   } else {
-    static bool attr = false; if (!attr) { FB_CUDA(cudaFuncSetAttribute(HistQuantKernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024)); attr = true; }
+    static PerDevice allowed; AllowSharedMemory(HistQuantKernel<false>, 200 * 1024, &allowed);
     HistQuantKernel<false><<<grid, kHistThreads, sm, s>>>(a);
   }
   FB_LAUNCHED(); FB_KERNEL_CHECK();
@@ -717,7 +717,7 @@ void LaunchHistConstructFloat(const HistArgs& a, cudaStream_t s) {
     return;
   }
   const size_t sm = static_cast<size_t>(a.max_part_bins) * 8 + static_cast<size_t>(a.num_groups) * 4;
-  static bool attr = false; if (!attr) { FB_CUDA(cudaFuncSetAttribute(HistFloatKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024)); attr = true; }
+  static PerDevice allowed; AllowSharedMemory(HistFloatKernel, 200 * 1024, &allowed);
   dim3 grid(a.total_blocks, a.num_parts);
   HistFloatKernel<<<grid, kHistThreads, sm, s>>>(a);
   FB_LAUNCHED(); FB_KERNEL_CHECK();

@@ -264,8 +264,8 @@ bool LaunchHistConstructQuantTC(const HistArgs& a, cudaStream_t s) {
                                CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (rc != CUDA_SUCCESS) { Log::Warning("tensor-core histogram: the gradient tensor map was refused (driver code %d)", static_cast<int>(rc)); return false; }
   }
-  static bool attr = false;
-  if (!attr) { FB_CUDA(cudaFuncSetAttribute(HistQuantTCKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmemBytes)); attr = true; }
+  static PerDevice allowed;
+  AllowSharedMemory(HistQuantTCKernel, kTcSmemBytes, &allowed);
   HistQuantTCKernel<<<a.total_blocks, kTcThreads, kTcSmemBytes, s>>>(a, rows_map, gh_map);
   FB_LAUNCHED(); FB_KERNEL_CHECK();
   return true;

@@ -94,8 +94,11 @@ size_t NodeMaskSharedBytes(const NodeMaskArgs& a) {
 void LaunchNodeMask(const NodeMaskArgs& a, cudaStream_t s) {
   if (a.num_children <= 0 || a.pool_size <= 0) return;
   const size_t sm = NodeMaskSharedBytes(a);
-  static size_t attr = 48 * 1024;
-  if (sm > attr) { FB_CUDA(cudaFuncSetAttribute(NodeMaskKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sm))); attr = sm; }
+  if (sm > 48 * 1024) {   // up to what a block may have at all
+    static PerDevice allowed;
+    cudaFuncAttributes attr; FB_CUDA(cudaFuncGetAttributes(&attr, NodeMaskKernel));
+    AllowSharedMemory(NodeMaskKernel, 227 * 1024 - static_cast<int>(attr.sharedSizeBytes), &allowed);
+  }
   NodeMaskKernel<<<a.num_children, kMaskThreads, sm, s>>>(a); FB_LAUNCHED(); FB_KERNEL_CHECK();
 }
 

@@ -318,8 +318,8 @@ bool DevicePredictTiled(const GBDT* gbdt, const void* device_data, int dtype, in
   const int nc = static_cast<int>(chunks.size());
 #define FB_TILED_P(T, LEAF, PLAIN)                                                                                                 \
   {                                                                                                                                \
-    static bool attr = false;                                                                                                      \
-    if (!attr) { FB_CUDA(cudaFuncSetAttribute(PredictTiledKernel<T, LEAF, PLAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPredictSmem)); attr = true; } \
+    static PerDevice allowed;                                                                                                      \
+    AllowSharedMemory(PredictTiledKernel<T, LEAF, PLAIN>, kPredictSmem, &allowed);                                                 \
     PredictTiledKernel<T, LEAF, PLAIN><<<grid, kPredictThreads, smem, s>>>(d_blob, d_chunks, nc, chunk_bytes, d_used, nu, static_cast<const T*>(device_data), nrow, ncol, \
                                                                            row_major ? 1 : 0, log_rows, K, num_trees, inv_avg, out_device);   \
   }

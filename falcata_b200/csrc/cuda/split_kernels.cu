@@ -583,16 +583,13 @@ void LaunchFindSplits(const FindArgs& a, cudaStream_t s, const CtrlArgs* tail_ct
   dim3 grid(a.num_children, std::max(1, (nf + warps - 1) / warps));
   size_t sm = static_cast<size_t>(warps) * (a.has_categorical ? std::max<size_t>(sizeof(CatScratch), a.quant ? kStagedBytes<true> : kStagedBytes<false>) : (a.quant ? kStagedBytes<true> : kStagedBytes<false>));
   if (a.fused_tail) sm = std::max(sm, sizeof(TailShared));
-  static bool attr = false;
-  if (!attr) {
-    constexpr int kMaxSmem = static_cast<int>(std::max(sizeof(CatScratch) * (kFindThreads / 32), sizeof(TailShared)));
-    static_assert(kMaxSmem <= 220 * 1024 && sizeof(CatScratch) >= kStagedBytes<false>, "a block of categorical warps fits an SM");
-    FB_CUDA(cudaFuncSetAttribute(FindSplitsKernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem));
-    FB_CUDA(cudaFuncSetAttribute(FindSplitsKernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem));
-    attr = true;
-  }
+  constexpr int kMaxSmem = static_cast<int>(std::max(sizeof(CatScratch) * (kFindThreads / 32), sizeof(TailShared)));
+  static_assert(kMaxSmem <= 220 * 1024 && sizeof(CatScratch) >= kStagedBytes<false>, "a block of categorical warps fits an SM");
+  static PerDevice allowed[2];
+  const auto kernel = a.quant ? FindSplitsKernel<true> : FindSplitsKernel<false>;
+  AllowSharedMemory(kernel, kMaxSmem, &allowed[a.quant ? 1 : 0]);
   const CtrlArgs ca = tail_ctrl != nullptr ? *tail_ctrl : CtrlArgs();
-  LaunchChained(a.wait.world <= 1 && a.wait_best.world <= 1, a.quant ? FindSplitsKernel<true> : FindSplitsKernel<false>, grid, dim3(warps * 32), sm, s, a, ca);
+  LaunchChained(a.wait.world <= 1 && a.wait_best.world <= 1, kernel, grid, dim3(warps * 32), sm, s, a, ca);
   FB_LAUNCHED(); FB_KERNEL_CHECK();
 }
 

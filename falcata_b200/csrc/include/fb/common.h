@@ -19,6 +19,7 @@
 #include <string>
 #include <vector>
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <map>
 #include <mutex>
@@ -76,6 +77,17 @@ class Log {
 int RowThreads(long long rows);
 // the team size of every parallel region that is not serial: the OpenMP thread limit
 int TeamThreads();
+
+// The set of devices something was done on, for host threads that may ask at the same time. A kernel's shared-memory limit
+// is set per device: a flag for the whole process would leave a second GPU with the default of 48 KB. (A device past the 64
+// of the set never counts as done; two threads that ask at once may both do it.)
+class PerDevice {
+ public:
+  bool Done(int device) const { return device >= 0 && device < 64 && ((done_.load(std::memory_order_acquire) >> device) & 1u) != 0; }
+  void SetDone(int device) { if (device >= 0 && device < 64) done_.fetch_or(1ull << device, std::memory_order_release); }
+ private:
+  std::atomic<unsigned long long> done_{0};
+};
 
 // Debugging switches read once from the environment.
 //   FALCATA_DEBUG=diag,dump,sync,canary,maxsplits=N   canary: guard words behind every region of the symmetric heap,

@@ -322,7 +322,20 @@ static void TestForcedSplitFile() {
   CHECK(LoadForcedSplitsFile("").empty());
 }
 
+// Per-device flags: a GPU's flag says nothing about another GPU.
+static void TestPerDevice() {
+  PerDevice done;
+  CHECK(!done.Done(0) && !done.Done(63));
+  done.SetDone(0);
+  CHECK(done.Done(0) && !done.Done(1) && !done.Done(63));
+  done.SetDone(63); done.SetDone(1);
+  CHECK(done.Done(0) && done.Done(1) && done.Done(63) && !done.Done(2));
+  done.SetDone(64); done.SetDone(-1);
+  CHECK(!done.Done(64) && !done.Done(-1) && !done.Done(2));
+}
+
 int main() {
+  TestPerDevice();
   TestBinFindingInvariants();
   TestCategoricalBins();
   TestLinearLeaves();

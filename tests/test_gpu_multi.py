@@ -30,6 +30,26 @@ def _run(world, out, extra=()):
 
 
 @pytest.mark.skipif(torch.cuda.device_count() < 2, reason="needs 2 GPUs")
+def test_one_process_trains_and_predicts_on_two_gpus_in_turn():
+    """Kernels that need more than 48 KB of shared memory ask for it on every device they run on."""
+    import falcata_b200 as fb
+    from util import make_binary, model_body
+
+    X, y = make_binary(20000, 20)
+    bodies = []
+    try:
+        for dev in (0, 1):
+            torch.cuda.set_device(dev)
+            for quant in ("none", "stochastic"):
+                bst = fb.train({"objective": "binary", "num_leaves": 31, "max_bin": 63, "verbosity": -1, "quant_mode": quant, "device_type": "cuda"}, fb.Dataset(X, y), 3)
+                bodies.append((model_body(bst.model_to_string()), bst.predict(torch.from_numpy(X).cuda(), raw_score=True).cpu()))
+    finally:
+        torch.cuda.set_device(0)
+    for quant in (0, 1):
+        assert bodies[quant][0] == bodies[2 + quant][0] and torch.equal(bodies[quant][1], bodies[2 + quant][1])
+
+
+@pytest.mark.skipif(torch.cuda.device_count() < 2, reason="needs 2 GPUs")
 @pytest.mark.parametrize("quant", ["stochastic", "fixedpoint"])
 def test_bit_identical_across_gpu_counts(tmp_path, quant):
     extra = ("--quant", quant)
