@@ -260,6 +260,7 @@ struct PartArgs {
   const LevelCtrl* ctrl;     // non-null: num_splits / total_chunks come from the device controller
   unsigned long long* chunk_words;   // non-null: one launch per level; [chunks] look-back words, valid when they carry `epoch`
   unsigned int epoch;                // one-launch form: differs from that of every earlier launch on the same words (never 0)
+  int rights_down;                   // three-launch form: rights from the window's end downwards, the order of the one-launch form (0: stable)
   int identity;                      // one-launch form: the windows hold the rows in order (root of an unbagged tree), idx is not read
   // ---- feature-parallel bitmap broadcast (bc_world > 1) ----
   // Every rank holds all rows but only the histograms of the features it owns. The rank that owns a

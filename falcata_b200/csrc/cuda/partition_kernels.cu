@@ -3,11 +3,13 @@
 // the left count before it from its predecessors' published counts (decoupled look-back) and writes the row ids it still
 // holds in registers: lefts upwards from the window's start, rights downwards from its end, so the total is not needed. A
 // leaf's rows stay in ascending or descending row order. The last chunk of a split writes the children's records.
-// Three launches (feature-parallel, plan fused_scan:off, the kernel-level entry points; stable in both children):
+// Three launches (feature-parallel, host-driven level loop, plan fused_scan:off; the kernel-level entry points). The order of a
+// leaf's rows is the order in which its fp32 sums are added, so training asks for the one-launch form's order here too
+// (rights_down) and its models do not depend on the form; the entry points are stable in both children.
 //   flags   : per 2048-row chunk, go-left ballot words + left count
 //   scan    : per split, exclusive scan of its chunks' counts; child windows, leaf records and the
 //             construct task of the smaller child are written here (no host round trip)
-//   scatter : popc-ranked stable scatter
+//   scatter : popc-ranked scatter
 // Parity: src/treelearner/cuda/cuda_data_partition.cu:L1380-1433 (ballot bit vectors, flat grid),
 // L1479 (per-split scan), L1562-1617 (stable scatter), L1681-1840 (tree-structure bookkeeping),
 // L1921 (copy back — removed here by the ping-pong buffers).
@@ -289,7 +291,10 @@ __global__ void __launch_bounds__(kPartThreads) PartitionScatterKernel(PartArgs 
     const int lefts_before_me = s_pref[w] + __popc(word & ((1u << lane) - 1u));
     const int row = src[pos];
     if ((word >> lane) & 1u) dst[left_before + lefts_before_me] = row;
-    else dst[total_left + right_before + (in_chunk - lefts_before_me)] = row;
+    else {
+      const int rights = right_before + (in_chunk - lefts_before_me);   // rights of the split before this row
+      dst[a.rights_down ? sp.count - 1 - rights : total_left + rights] = row;
+    }
   }
 }
 

@@ -1,7 +1,9 @@
 """Plan tuner with a wisdom file.
 
-Every ``cuda_plan`` switch except the quantizer ones chooses between implementations that produce the same model, so
-they can be chosen by the clock. ``tune`` times a few boosting rounds of the actual training job per candidate plan
+Every ``cuda_plan`` switch except the quantizer ones chooses between implementations of the same sums, so they can be
+chosen by the clock: with integer histograms the models are byte-identical. With fp32 histograms (``quant_mode=none``) of at
+most 64 bins only ``hist_float_red`` changes a model, by the rounding of its sums; fp32 histograms of more bins are added in no
+fixed order and differ by rounding from run to run, whatever the plan. ``tune`` times a few boosting rounds of the actual training job per candidate plan
 (coordinate descent over the switches: flip one, keep the flip if it is faster by more than the noise margin), returns
 the fastest plan and remembers it in a small JSON "wisdom" file keyed by the workload's shape and the device, so that
 the next training of the same shape on the same kind of GPU starts from the known-best plan:
@@ -22,7 +24,7 @@ import time
 from pathlib import Path
 from typing import Any, Callable, Dict, List, Optional
 
-# switches whose two settings give byte-identical models (the quantizer switches robust_scale / quant_ef change the model)
+# switches whose two settings give byte-identical models on integer histograms (the quantizer switches robust_scale / quant_ef change the model)
 TUNABLE = ["hist_lane_red", "fused_tail", "fused_scan", "col_major_part", "bulk_root", "gh_in_row", "compact_view", "pack4", "hist_float_red"]
 _DEFAULT_ON = {"hist_lane_red": True, "fused_tail": True, "fused_scan": True, "col_major_part": True, "bulk_root": True, "gh_in_row": False, "compact_view": True,
                "pack4": True, "hist_float_red": False}

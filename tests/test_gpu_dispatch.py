@@ -80,6 +80,17 @@ def test_one_launch_partition_gives_the_same_model(n, extra):
     assert models[0] == models[1]
 
 
+@pytest.mark.parametrize("flip", ["fused_scan:off", "fused_tail:off,fused_scan:off", "device_controller:off"])
+@pytest.mark.parametrize("max_bin", [15, 63])
+@pytest.mark.parametrize("n", [2049, 30000])
+def test_fp32_sums_do_not_depend_on_the_partition_form(n, max_bin, flip):
+    """fp32 histograms of at most 64 bins are sums in the order of a leaf's rows: every form of the partition leaves the same order."""
+    X, y = make_binary(n, 20)
+    p = {"objective": "binary", "num_leaves": 63, "max_bin": max_bin, "verbosity": -1, "quant_mode": "none", "device_type": "cuda", "min_data_in_leaf": 5}
+    models = [model_body(fb.train(dict(p, cuda_plan=plan), fb.Dataset(X, y), 8).model_to_string()) for plan in ("auto", "auto," + flip)]
+    assert models[0] == models[1]
+
+
 @pytest.mark.parametrize("features", [1, 8, 9, 16, 17, 40])
 @pytest.mark.parametrize("max_bin", [7, 31, 32, 33, 64, 65, 127, 255])
 def test_split_search_agrees_with_the_host(features, max_bin):
