@@ -481,7 +481,7 @@ Tree* CudaEngine::TrainTree(int class_id, int tree_index) {
     ChildInit* ci = reinterpret_cast<ChildInit*>(hb + sizeof(PartSplit) * S);
     FindChild* fc = reinterpret_cast<FindChild*>(hb + (sizeof(PartSplit) + sizeof(ChildInit)) * S);
     long long total_rows = 0; for (int l : cand) total_rows += host_leaves_[l].count;
-    ha.rows_per_block = ChooseRowsPerBlock(total_rows);
+    ha.rows_per_block = quant_ ? ChooseRowsPerBlock(total_rows) : rpb;   // fp32 sums depend on where blocks end: as with the device controller
     int chunk_cursor = 0, block_cursor = 0;
     std::vector<int>& next = *next_out; next.clear();
     for (int s = 0; s < S; ++s) {

@@ -82,9 +82,10 @@ def test_one_launch_partition_gives_the_same_model(n, extra):
 
 @pytest.mark.parametrize("flip", ["fused_scan:off", "fused_tail:off,fused_scan:off", "device_controller:off"])
 @pytest.mark.parametrize("max_bin", [15, 63])
-@pytest.mark.parametrize("n", [2049, 30000])
+@pytest.mark.parametrize("n", [2049, 30000, 150001])
 def test_fp32_sums_do_not_depend_on_the_partition_form(n, max_bin, flip):
-    """fp32 histograms of at most 64 bins are sums in the order of a leaf's rows: every form of the partition leaves the same order."""
+    """fp32 histograms of at most 64 bins are sums in the order of a leaf's rows: every form of the partition leaves the same
+    order, and every level loop ends its blocks at the same rows."""
     X, y = make_binary(n, 20)
     p = {"objective": "binary", "num_leaves": 63, "max_bin": max_bin, "verbosity": -1, "quant_mode": "none", "device_type": "cuda", "min_data_in_leaf": 5}
     models = [model_body(fb.train(dict(p, cuda_plan=plan), fb.Dataset(X, y), 8).model_to_string()) for plan in ("auto", "auto," + flip)]
