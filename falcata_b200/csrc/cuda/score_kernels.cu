@@ -15,13 +15,20 @@ namespace {
 
 // score[row] += v for the rows of a leaf's window, walked by gridDim.y blocks. A row is in one window, so the reduction adds
 // (nothing comes back to the SM: 32 scattered sectors per instruction once instead of twice) do not depend on their order.
-// (A global reduction add flushes a subnormal sum, below 1.2e-38, to zero.)
+// A global reduction add takes subnormal numbers as zero, in and out. From |v| = 2^-100 on that changes nothing: a subnormal score
+// is less than half a unit in v's last place (2^-125 at least, also just below a power of two), and a sum that is not zero is
+// a multiple of 2^-125 or more. Smaller values, zero and NaN take load, add and store.
 // Measured at 11M rows and 255 leaves: 172 us with load, add and store, 62 us.
 __device__ __forceinline__ void AddToWindow(const LeafInfo& L, float v, const int* __restrict__ idx0, const int* __restrict__ idx1, float* __restrict__ score) {
   const int* idx = (L.buffer ? idx1 : idx0) + L.begin;
   const int stride = gridDim.y * blockDim.x;
+  const int first = blockIdx.y * blockDim.x + threadIdx.x;
+  if (fabsf(v) >= 0x1p-100f) {
 #pragma unroll 4
-  for (int p = blockIdx.y * blockDim.x + threadIdx.x; p < L.count; p += stride) atomicAdd(score + idx[p], v);
+    for (int p = first; p < L.count; p += stride) atomicAdd(score + idx[p], v);
+  } else {
+    for (int p = first; p < L.count; p += stride) score[idx[p]] += v;
+  }
 }
 __global__ void AddLeafOutputsKernel(const LeafInfo* __restrict__ leaves, const double* __restrict__ leaf_value, const int* __restrict__ idx0,
                                      const int* __restrict__ idx1, float* __restrict__ score) {

@@ -92,6 +92,17 @@ def test_fp32_sums_do_not_depend_on_the_partition_form(n, max_bin, flip):
     assert models[0] == models[1]
 
 
+@pytest.mark.parametrize("grow", ["level", "leaf"])
+@pytest.mark.parametrize("rate", [1e-39, 3e-38, 2.0 ** -100, 1e-20])
+def test_leaf_outputs_of_any_size_reach_the_scores(rate, grow):
+    """Subnormal leaf outputs and scores, and outputs on both sides of the size from which reduction adds are used."""
+    X, y = make_binary(3000, 5)
+    p = {"objective": "binary", "num_leaves": 15, "verbosity": -1, "quant_mode": "stochastic", "device_type": "cuda", "learning_rate": rate, "boost_from_average": False, "grow_policy": grow}
+    bst = fb.train(p, fb.Dataset(X, y), 1, keep_training_booster=True)
+    expected = bst.predict(X, raw_score=True).astype(np.float32)   # one tree on scores of zero: its outputs, rounded once
+    assert np.count_nonzero(expected) == len(expected) and np.array_equal(bst.train_score_tensor().cpu().numpy().reshape(-1), expected)
+
+
 @pytest.mark.parametrize("features", [1, 8, 9, 16, 17, 40])
 @pytest.mark.parametrize("max_bin", [7, 31, 32, 33, 64, 65, 127, 255])
 def test_split_search_agrees_with_the_host(features, max_bin):
