@@ -644,16 +644,16 @@ static LaneGeometry LaneShape(bool red, int sub_rows, int nb, bool flt) {
   if (const char* e = std::getenv("FALCATA_LANE_WARPS")) g.warps = std::atoi(e);
   if (g.warps < 4 || g.warps > 32) Log::Fatal("FALCATA_LANE_WARPS must be within 4..32");
   const size_t stage_bytes = static_cast<size_t>(g.warps) * g.stages * (32 * (32 + (flt ? 8 : 4)) + 8);
-  if (stage_bytes + tile_bytes > budget) Log::Fatal("lane histogram: a %d-bin tile does not fit beside the stages of %d warps", nb, g.warps);
-  const int fit = static_cast<int>((budget - stage_bytes) / tile_bytes);
+  const size_t beside = std::max(stage_bytes, FlushBytes(nb, flt));   // the flush takes the stages' place
+  if (beside + tile_bytes > budget) Log::Fatal("lane histogram: a %d-bin tile does not fit beside the stages of %d warps", nb, g.warps);
+  const int fit = static_cast<int>((budget - beside) / tile_bytes);
   int tiles = 1;
   if (!red) tiles = g.warps;   // the load-add-store form needs a tile per warp
   else for (int t = 1; t <= g.warps; ++t) if (g.warps % t == 0 && t <= fit && (!wide || t <= 4)) tiles = t;
   if (const char* e = std::getenv("FALCATA_LANE_SHARE")) { const int ss = std::atoi(e); if (red && ss >= 1 && g.warps % ss == 0) tiles = g.warps / ss; }
   if (tiles > fit) Log::Fatal("lane histogram: %d tiles of %d bins do not fit beside the stages of %d warps", tiles, nb, g.warps);
   g.share = g.warps / tiles;
-  g.smem = tile_bytes * tiles + std::max(stage_bytes, FlushBytes(nb, flt));
-  if (g.smem > budget) Log::Fatal("lane histogram: %d tiles of %d bins leave no room for the block's flush", tiles, nb);
+  g.smem = tile_bytes * tiles + beside;
   g.red = red;
   return g;
 }

@@ -53,6 +53,26 @@ def test_lane_construct(n, groups, nb, rpb):
                 assert bool(((out[:, k] - _reference(rows, groups, nb, gh[:, k], sub)).abs() <= bound).all())
 
 
+@pytest.mark.parametrize("warps,quant,nb", [(6, False, 256), (9, False, 200), (12, True, 256), (6, True, 256)])
+def test_lane_construct_with_few_warps(monkeypatch, warps, quant, nb):
+    """Few warps stage little: the block's flush, which takes the stages' place, then decides how many tiles fit."""
+    from falcata_b200 import ops
+    monkeypatch.setenv("FALCATA_LANE_WARPS", str(warps))
+    gen = torch.Generator(device="cuda"); gen.manual_seed(warps)
+    n, groups = 5003, 33
+    rows = _rows(n, groups, nb, gen)
+    if quant:
+        gi = torch.randint(-32, 33, (n,), generator=gen, device="cuda", dtype=torch.int32)
+        hi = torch.randint(0, 65, (n,), generator=gen, device="cuda", dtype=torch.int32)
+        out = ops.histogram(rows, (gi << 16) | hi, [nb] * groups, quant=True, quant_bins=64, rows_per_block=512, lane_mode=1)
+        assert torch.equal(out[:, 0], _reference(rows, groups, nb, gi).long()) and torch.equal(out[:, 1], _reference(rows, groups, nb, hi).long())
+    else:
+        gh = torch.randint(-8, 9, (n, 2), generator=gen, device="cuda").float() / 8   # sums of a coarse grid: exact in fp32
+        out = ops.histogram(rows, gh, [nb] * groups, quant=False, rows_per_block=512, lane_mode=2)
+        for k in range(2):
+            assert torch.equal(out[:, k], _reference(rows, groups, nb, gh[:, k]))
+
+
 @pytest.mark.parametrize("n", [1, 3, 4, 5, 1023, 148 * 8 * 256 * 4 + 3])
 def test_quantize_walks_every_row(n):
     from falcata_b200 import ops
