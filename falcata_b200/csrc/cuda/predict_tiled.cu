@@ -15,11 +15,13 @@
 // more than 65534 used features, or trees above 4096 leaves take the general one-thread-per-row kernel.
 #include <cuda_fp16.h>
 #include <cuda_pipeline.h>
+#include <omp.h>
 
 #include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <limits>
+#include <memory>
 #include <vector>
 
 #include "engine.h"
@@ -38,6 +40,7 @@ static_assert(sizeof(PackedNode) == 8, "8-byte nodes");
 constexpr int kPredictThreads = 512;        // threads of a block = rows of its tile x tree slices
 constexpr int kMaxTileRows = 256;
 constexpr int kTreeBytes = 32 * 1024;       // a tree and its root word must fit this much; also the smaller chunk size
+constexpr int kMaxTreeSplits = kTreeBytes / 16;   // two 8-byte nodes a split
 constexpr int kPredictSmem = 220 * 1024;
 constexpr unsigned int kLeafType = 3;
 constexpr unsigned int kChildMask = 0xFFF8u;
@@ -188,7 +191,9 @@ PredictTiledKernel(const unsigned char* __restrict__ blob, const ChunkDesc* __re
 
 // Nodes of one tree in sibling-adjacent order, root first, then every split's two children next to each other, placed at
 // byte `base` of their chunk. slot_base: slot of the tile's first feature row; leaf_slot: slot of the row of -infinity.
-void PackTree(const Tree& T, const std::vector<int>& slot_of_feature, int slot_base, int leaf_slot, bool leaf_index, int base, PackedNode* out) {
+// queue: room for the tree's splits (this runs inside a parallel region, which no exception may leave: nothing is allocated here).
+struct QueuedSplit { int id, pos; };   // host id, packed position
+void PackTree(const Tree& T, const std::vector<int>& slot_of_feature, int slot_base, int leaf_slot, bool leaf_index, int base, QueuedSplit* queue, PackedNode* out) {
   auto offset = [&](int pos) { return static_cast<unsigned int>(base + pos * static_cast<int>(sizeof(PackedNode))); };
   auto place = [&](int id, int pos) {   // host ids: >= 0 split, < 0 leaf ~id
     if (id >= 0) return;
@@ -196,27 +201,26 @@ void PackTree(const Tree& T, const std::vector<int>& slot_of_feature, int slot_b
     out[pos].meta = (static_cast<unsigned int>(leaf_slot) << 16) | offset(pos) | (kLeafType << 1);
   };
   if (T.num_leaves <= 1) { place(~0, 0); return; }
-  // splits in breadth-first order: (host id, packed position)
-  std::vector<std::pair<int, int>> queue; queue.reserve(T.num_leaves - 1);
-  queue.emplace_back(0, 0);
-  int next_free = 1;
-  for (size_t qi = 0; qi < queue.size(); ++qi) {
-    const int id = queue[qi].first, left_pos = next_free;
+  int queued = 0, next_free = 1;   // splits in breadth-first order
+  queue[queued++] = {0, 0};
+  for (int qi = 0; qi < queued; ++qi) {
+    const int id = queue[qi].id, left_pos = next_free;
     next_free += 2;
     float thr = static_cast<float>(T.threshold[id]);
     // keep "v <= threshold" exact for float inputs: round the double threshold DOWN to float
     if (static_cast<double>(thr) > T.threshold[id]) thr = std::nextafterf(thr, -std::numeric_limits<float>::infinity());
-    PackedNode& nd = out[queue[qi].second];
+    PackedNode& nd = out[queue[qi].pos];
     nd.value = thr;
     nd.meta = (static_cast<unsigned int>(slot_base + slot_of_feature[T.split_feature[id]]) << 16) | offset(left_pos) |
               (static_cast<unsigned int>(Tree::MissingTypeOf(T.decision_type[id])) << 1) | ((T.decision_type[id] & kDefaultLeftMask) ? 1u : 0u);
     const int child[2] = {T.left_child[id], T.right_child[id]};
-    for (int c = 0; c < 2; ++c) { if (child[c] >= 0) queue.emplace_back(child[c], left_pos + c); else place(child[c], left_pos + c); }
+    for (int c = 0; c < 2; ++c) { if (child[c] >= 0) queue[queued++] = {child[c], left_pos + c}; else place(child[c], left_pos + c); }
   }
 }
 
 // What the packed form asks of a tree, and what the tree brings: the features it reads and whether it has missing-aware nodes.
-bool ScanTree(const Tree& T, bool leaf_index, std::vector<char>* uses, bool* plain) {
+// uses: a flag per feature. (Inside a parallel region, like PackTree.)
+bool ScanTree(const Tree& T, bool leaf_index, char* uses, int num_features, bool* plain) {
   if (T.is_linear || T.num_leaves > 4096) return false;
   if ((std::max(1, 2 * T.num_leaves - 1)) * sizeof(PackedNode) + 32 > static_cast<size_t>(kTreeBytes)) return false;   // larger than a buffer
   if (!leaf_index) for (int l = 0; l < std::max(1, T.num_leaves); ++l) if (std::isnan(T.leaf_value[l])) return false;    // a leaf holds its place by -infinity <= value
@@ -224,8 +228,8 @@ bool ScanTree(const Tree& T, bool leaf_index, std::vector<char>* uses, bool* pla
     if (T.decision_type[s] & kCategoricalMask) return false;
     if (Tree::MissingTypeOf(T.decision_type[s]) != 0) *plain = false;
     const int f = T.split_feature[s];
-    if (f < 0 || f >= static_cast<int>(uses->size())) return false;
-    (*uses)[f] = 1;
+    if (f < 0 || f >= num_features) return false;
+    uses[f] = 1;
   }
   return true;
 }
@@ -245,18 +249,15 @@ bool DevicePredictTiled(const GBDT* gbdt, const void* device_data, int dtype, in
   const bool parallel = forest_nodes > (1 << 15);
   // features the forest reads, in ascending order
   const size_t nfeat = std::max(1, gbdt->max_feature_idx_ + 1);
-  std::vector<char> uses(nfeat, 0);
+  const int team = parallel ? TeamThreads() : 1;
+  std::vector<char> uses(team * nfeat, 0);   // a row per thread
   bool plain = true, covered = true;   // plain: no node with a missing type - NaN reads as 0 everywhere, zero is an ordinary value
-#pragma omp parallel num_threads(parallel ? TeamThreads() : 1)
-  {
-    std::vector<char> mine(nfeat, 0); bool my_plain = true, my_covered = true;
-#pragma omp for schedule(static) nowait
-    for (int t = 0; t < num_trees; ++t) my_covered = my_covered && ScanTree(*gbdt->models_[first_tree + t], leaf_index, &mine, &my_plain);
-#pragma omp critical(fb_predict_scan)
-    { for (size_t f = 0; f < nfeat; ++f) uses[f] |= mine[f]; plain = plain && my_plain; covered = covered && my_covered; }
-  }
+#pragma omp parallel for schedule(static) num_threads(team) reduction(&& : plain, covered)
+  for (int t = 0; t < num_trees; ++t)
+    covered = covered && ScanTree(*gbdt->models_[first_tree + t], leaf_index, uses.data() + omp_get_thread_num() * nfeat, static_cast<int>(nfeat), &plain);
   if (!covered) return false;
   std::vector<int> slot_of_feature(nfeat, -1), used;
+  for (int k = 1; k < team; ++k) for (size_t f = 0; f < nfeat; ++f) uses[f] |= uses[k * nfeat + f];
   for (size_t f = 0; f < nfeat; ++f) if (uses[f]) { slot_of_feature[f] = static_cast<int>(used.size()); used.push_back(static_cast<int>(f)); }
   if (used.empty()) used.push_back(0);
   const int nu = static_cast<int>(used.size());
@@ -301,11 +302,13 @@ bool DevicePredictTiled(const GBDT* gbdt, const void* device_data, int dtype, in
   std::vector<unsigned char> staged(blob_at + bytes);
   memcpy(staged.data() + chunks_at, chunks.data(), chunks.size() * sizeof(ChunkDesc));
   memcpy(staged.data() + used_at, used.data(), used.size() * sizeof(int));
-#pragma omp parallel for schedule(static) num_threads(parallel ? TeamThreads() : 1)
+  const std::unique_ptr<QueuedSplit[]> queues(new QueuedSplit[static_cast<size_t>(team) * kMaxTreeSplits]);
+#pragma omp parallel for schedule(static) num_threads(team)
   for (int t = 0; t < num_trees; ++t) {
     const ChunkDesc& d = chunks[place[t].chunk];
     unsigned char* chunk = staged.data() + blob_at + d.offset;
-    PackTree(*gbdt->models_[first_tree + t], slot_of_feature, slot_base, slot_base + nu, leaf_index, place[t].base, reinterpret_cast<PackedNode*>(chunk + place[t].base));
+    PackTree(*gbdt->models_[first_tree + t], slot_of_feature, slot_base, slot_base + nu, leaf_index, place[t].base,
+             queues.get() + static_cast<size_t>(omp_get_thread_num()) * kMaxTreeSplits, reinterpret_cast<PackedNode*>(chunk + place[t].base));
     reinterpret_cast<int*>(chunk + d.roots)[place[t].pos] = place[t].base;
   }
   DevBuf<unsigned char> forest;

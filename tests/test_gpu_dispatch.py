@@ -176,6 +176,28 @@ def test_search_of_bundled_features_agrees_with_the_host(levels, quant, zero_as_
     assert any(int(t) < len(columns) for line in bodies[0].splitlines() if line.startswith("split_feature=") for t in line.split("=")[1].split())
 
 
+def test_several_threads_predict_at_once():
+    """Forests large enough to be packed by a team of threads, predicted by several threads at a time: each gets its own answer."""
+    import threading
+    rng = np.random.RandomState(3)
+    X = rng.randn(4000, 30).astype(np.float32)
+    boosters = [_forest(150 + 20 * k, 127, 30, k, X) for k in range(3)]   # about 38k nodes and more
+    x = torch.from_numpy(X[:500]).cuda()
+    alone = [(b.predict(x, raw_score=True).clone(), b.predict(x, pred_leaf=True).clone()) for b in boosters]
+    same = [False] * 6
+
+    def work(i):
+        b, (score, leaf) = boosters[i % 3], alone[i % 3]
+        same[i] = all(torch.equal(b.predict(x, raw_score=True), score) and torch.equal(b.predict(x, pred_leaf=True), leaf) for _ in range(5))
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(6)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert all(same)
+
+
 def _forest(trees, leaves, features, seed, X):
     rng = np.random.RandomState(seed)
     y = (X[:, 0] + rng.randn(len(X)) > 0).astype(np.float32)
