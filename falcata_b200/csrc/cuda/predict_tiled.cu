@@ -162,7 +162,7 @@ PredictTiledKernel(const unsigned char* __restrict__ blob, const ChunkDesc* __re
 #pragma unroll
           for (int q = 0; q < kWalks; ++q) {
             unsigned int next = (nd[q].meta & kChildMask) | buf;
-            // a leaf stays where it is: -infinity goes left, and its left child is itself
+            // a leaf stays where it is: -infinity goes left, and its left child is itself (a NaN leaf: right, and so is its right child)
             if (!GoLeft<PLAIN>(v[q], nd[q].value, nd[q].meta)) next += 8u;
             nd[q] = *reinterpret_cast<const PackedNode*>(smem + next);
           }
@@ -198,7 +198,9 @@ void PackTree(const Tree& T, const std::vector<int>& slot_of_feature, int slot_b
   auto place = [&](int id, int pos) {   // host ids: >= 0 split, < 0 leaf ~id
     if (id >= 0) return;
     if (leaf_index) { const int leaf = ~id; std::memcpy(&out[pos].value, &leaf, sizeof(int)); } else out[pos].value = static_cast<float>(T.leaf_value[~id]);
-    out[pos].meta = (static_cast<unsigned int>(leaf_slot) << 16) | offset(pos) | (kLeafType << 1);
+    // -infinity goes left at every value but NaN: a NaN leaf's left child is the node before it, so that its right one is itself
+    const bool nan = !leaf_index && std::isnan(T.leaf_value[~id]);
+    out[pos].meta = (static_cast<unsigned int>(leaf_slot) << 16) | offset(nan ? pos - 1 : pos) | (kLeafType << 1);
   };
   if (T.num_leaves <= 1) { place(~0, 0); return; }
   int queued = 0, next_free = 1;   // splits in breadth-first order
@@ -223,7 +225,7 @@ void PackTree(const Tree& T, const std::vector<int>& slot_of_feature, int slot_b
 bool ScanTree(const Tree& T, bool leaf_index, char* uses, int num_features, bool* plain) {
   if (T.is_linear || T.num_leaves > 4096) return false;
   if ((std::max(1, 2 * T.num_leaves - 1)) * sizeof(PackedNode) + 32 > static_cast<size_t>(kTreeBytes)) return false;   // larger than a buffer
-  if (!leaf_index) for (int l = 0; l < std::max(1, T.num_leaves); ++l) if (std::isnan(T.leaf_value[l])) return false;    // a leaf holds its place by -infinity <= value
+  if (!leaf_index && T.num_leaves <= 1 && std::isnan(T.leaf_value[0])) return false;   // no node before it to lead to
   for (int s = 0; s < T.num_leaves - 1; ++s) {
     if (T.decision_type[s] & kCategoricalMask) return false;
     if (Tree::MissingTypeOf(T.decision_type[s]) != 0) *plain = false;

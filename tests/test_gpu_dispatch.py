@@ -176,6 +176,26 @@ def test_search_of_bundled_features_agrees_with_the_host(levels, quant, zero_as_
     assert any(int(t) < len(columns) for line in bodies[0].splitlines() if line.startswith("split_feature=") for t in line.split("=")[1].split())
 
 
+@pytest.mark.parametrize("missing", [False, True])
+def test_nan_leaf_outputs(missing):
+    """Rows that reach a NaN leaf get NaN, all others the same bits as without it: the same kernel adds them in the same order."""
+    rng = np.random.RandomState(9)
+    X = rng.randn(4000, 12).astype(np.float32)
+    if missing:
+        X[rng.rand(*X.shape) < 0.1] = np.nan
+    bst = _forest(300, 31, 12, 2, X)
+    x = torch.from_numpy(X[:1500]).cuda()
+    before = bst.predict(x, raw_score=True).cpu().numpy().reshape(-1)
+    leaf = np.asarray(bst.predict(X[:1500], pred_leaf=True)).reshape(1500, -1)
+    hit = np.zeros(1500, dtype=bool)
+    for tree in (0, 7, 299):
+        bst.set_leaf_output(tree, int(leaf[tree, tree]), float("nan"))
+        hit |= leaf[:, tree] == leaf[tree, tree]
+    after = bst.predict(x, raw_score=True).cpu().numpy().reshape(-1)
+    assert 0 < hit.sum() < 1500 and np.isnan(after[hit]).all() and np.array_equal(after[~hit], before[~hit])
+    assert np.array_equal(bst.predict(x, pred_leaf=True).cpu().numpy().reshape(1500, -1), leaf)
+
+
 def test_several_threads_predict_at_once():
     """Forests large enough to be packed by a team of threads, predicted by several threads at a time: each gets its own answer."""
     import threading
