@@ -337,6 +337,9 @@ void LaunchAddTreeBinned(const DevTree& t, const uint8_t* rows, int row_stride, 
 // flags: bit0 default_left, bits1-2 missing type, bit3 leaf (threshold = value), bit4 categorical (threshold holds,
 // as an int, the offset of the node's category bitset in the forest's word array; bits 8.. = number of words)
 struct ForestNode { float threshold; int feature; int left; int right; int flags; };
+// What the tiled prediction kernel covers: leaves of a tree (8-byte nodes of one tree in a 32 KB chunk), features that the forest
+// uses (a 32-row tile of them beside the tree ring), and features for the leaf indices of double rows (a 256-row tile).
+constexpr int kTiledTreeLeaves = 2046, kTiledFeatures = 1215, kTiledFeaturesF64Leaf = 156;
 template <typename T>
 void LaunchPredictRaw(const ForestNode* nodes, const unsigned int* cat_words, const int* tree_root, int num_trees, int num_class, const T* data, int nrow, int ncol, bool row_major,
                       float* out /* [num_class x nrow] */, bool average, cudaStream_t s);

@@ -23,14 +23,15 @@ void DevicePredict(const GBDT* gbdt, const void* device_data, int dtype, int32_t
   const int use = num_iter > 0 ? std::min(num_iter, iters - start_iter) : iters - start_iter;
   if (ncol <= gbdt->max_feature_idx_) Log::Fatal("The number of features in data (%d) is not the same as it was in training data (%d)", ncol, gbdt->max_feature_idx_ + 1);
   // the tiled kernel (rows staged in shared memory, trees streamed through it) covers numerical forests; everything
-  // else - categorical splits, very wide or very deep forests - walks the general node array below
+  // else - categorical splits, very wide forests or very large trees - walks the general node array below
   bool tiled = false;
   if (use > 0 && std::getenv("FALCATA_PREDICT_GENERAL") == nullptr) {
     const float inv = (gbdt->average_output_ && use > 0) ? 1.f / use : 1.f;
     tiled = DevicePredictTiled(gbdt, device_data, dtype, nrow, ncol, row_major, start_iter * K, use * K, K, predict_type == 2, inv, out_device, 0);
   }
   if (predict_type == 2) {
-    if (!tiled) Log::Fatal("Leaf-index prediction on the device covers numerical forests of at most 4096 leaves per tree; predict on the host");
+    if (!tiled) Log::Fatal("Leaf-index prediction on the device covers numerical forests of at most %d leaves per tree that use at most %d features (double rows: %d); predict on the host",
+                          kTiledTreeLeaves, kTiledFeatures, kTiledFeaturesF64Leaf);
     return;
   }
   if (tiled) {

@@ -11,8 +11,9 @@
 // nodes of indices; 200k rows x 100 features, 500 trees of 127 leaves with missing values, 3.8 -> 2.1 ms.
 //
 // Parity: python-package/falcata/basic.py:L5112-5163 (device predict route: raw score, converted score, leaf index),
-// include/Falcata/tree.h:L361-439 (numerical decision with missing-value handling). Forests with categorical splits,
-// more than 65534 used features, or trees above 4096 leaves take the general one-thread-per-row kernel.
+// include/Falcata/tree.h:L361-439 (numerical decision with missing-value handling). Forests with categorical splits, a tree of
+// more than kTiledTreeLeaves leaves, or more than kTiledFeatures used features take the general one-thread-per-row kernel;
+// leaf indices of these, and of double rows with more than kTiledFeaturesF64Leaf used features, come from the host.
 #include <cuda_fp16.h>
 #include <cuda_pipeline.h>
 #include <omp.h>
@@ -38,10 +39,11 @@ struct PackedNode { float value; unsigned int meta; };
 static_assert(sizeof(PackedNode) == 8, "8-byte nodes");
 
 constexpr int kPredictThreads = 512;        // threads of a block = rows of its tile x tree slices
-constexpr int kMaxTileRows = 256;
 constexpr int kTreeBytes = 32 * 1024;       // a tree and its root word must fit this much; also the smaller chunk size
-constexpr int kMaxTreeSplits = kTreeBytes / 16;   // two 8-byte nodes a split
+constexpr int kMaxTreeSplits = kTiledTreeLeaves - 1;
+static_assert((2 * kTiledTreeLeaves - 1) * static_cast<int>(sizeof(PackedNode)) + 32 <= kTreeBytes, "the largest tree fits a chunk");
 constexpr int kPredictSmem = 220 * 1024;
+static_assert(2 * kTreeBytes + (kTiledFeatures + 1) * 32 * 4 + kPredictThreads * 8 <= kPredictSmem, "the widest forest fits a 32-row tile beside two chunks");
 constexpr unsigned int kLeafType = 3;
 constexpr unsigned int kChildMask = 0xFFF8u;
 constexpr int kWalks = 4;                   // tree walks a thread keeps in flight
@@ -223,8 +225,7 @@ void PackTree(const Tree& T, const std::vector<int>& slot_of_feature, int slot_b
 // What the packed form asks of a tree, and what the tree brings: the features it reads and whether it has missing-aware nodes.
 // uses: a flag per feature. (Inside a parallel region, like PackTree.)
 bool ScanTree(const Tree& T, bool leaf_index, char* uses, int num_features, bool* plain) {
-  if (T.is_linear || T.num_leaves > 4096) return false;
-  if ((std::max(1, 2 * T.num_leaves - 1)) * sizeof(PackedNode) + 32 > static_cast<size_t>(kTreeBytes)) return false;   // larger than a buffer
+  if (T.is_linear || T.num_leaves > kTiledTreeLeaves) return false;
   if (!leaf_index && T.num_leaves <= 1 && std::isnan(T.leaf_value[0])) return false;   // no node before it to lead to
   for (int s = 0; s < T.num_leaves - 1; ++s) {
     if (T.decision_type[s] & kCategoricalMask) return false;
@@ -263,8 +264,9 @@ bool DevicePredictTiled(const GBDT* gbdt, const void* device_data, int dtype, in
   for (size_t f = 0; f < nfeat; ++f) if (uses[f]) { slot_of_feature[f] = static_cast<int>(used.size()); used.push_back(static_cast<int>(f)); }
   if (used.empty()) used.push_back(0);
   const int nu = static_cast<int>(used.size());
-  // leaf indices have no general kernel to fall back to: the widest forest is the one of a 256-row tile beside two chunks
-  if (leaf_index && 2 * kTreeBytes + nu * kMaxTileRows * 4 > kPredictSmem) return false;
+  // the walk compares in fp32, which is exact for fp32 and half rows; the leaf of a double row next to a threshold can differ from
+  // the host's, which compares in double: wide forests, which only tiles of fewer rows hold, leave it to the host as they always did
+  if (leaf_index && dtype == kF64 && nu > kTiledFeaturesF64Leaf) return false;
   int dev = 0, sms = 0; FB_CUDA(cudaGetDevice(&dev)); FB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   // The tile: as many rows as fit beside two chunks (the forest streams through the ring once per tile), but no more than
   // leave every SM a tile; the threads that rows do not take walk other trees.

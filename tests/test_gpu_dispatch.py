@@ -1,5 +1,7 @@
 """Kernel variants that a rule on sizes selects, at the edges of the rule: the lane construct's block flush, the one-launch row
 partition, the split search, the per-row kernels of a round's set-up and the tile shapes of prediction."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -235,4 +237,39 @@ def test_predict_tiles_match_the_host(rows, features, trees, leaves):
     # leaf values and the sums are rounded to fp32 once each: 2^-23 of the largest partial sum, far below 1e-5
     for t in (torch.from_numpy(x).cuda(), torch.from_numpy(x.astype(np.float64)).cuda()):
         np.testing.assert_allclose(bst.predict(t, raw_score=True).cpu().numpy().reshape(-1), np.asarray(bst.predict(x, raw_score=True)).reshape(-1), rtol=1e-5, atol=1e-5)
-    assert np.array_equal(np.asarray(bst.predict(torch.from_numpy(x).cuda(), pred_leaf=True).cpu()).reshape(rows, -1), np.asarray(bst.predict(x, pred_leaf=True)).reshape(rows, -1))
+    host = np.asarray(bst.predict(x, pred_leaf=True)).reshape(rows, -1)
+    rc, leaf = _device_leaves(bst, torch.from_numpy(x).cuda(), trees)
+    assert rc == 0 and np.array_equal(leaf, host)
+
+
+def _device_leaves(bst, x, trees):
+    """Leaf indices by the device entry point itself: ``Booster.predict`` would take what the device refuses to the host."""
+    from falcata_b200.basic import _lib
+    out = torch.full((x.shape[0], trees), -1, dtype=torch.int32, device="cuda")
+    code = {torch.float32: 0, torch.float64: 1, torch.float16: 6}[x.dtype]
+    rc = _lib().FB_BoosterPredictForDeviceMat(bst._handle, ctypes.c_void_p(x.data_ptr()), code, ctypes.c_int32(x.shape[0]), ctypes.c_int32(x.shape[1]), 1, 2, 0, -1,
+                                              ctypes.c_void_p(out.data_ptr()))
+    return rc, out.cpu().numpy()
+
+
+@pytest.mark.parametrize("features", [156, 157, 330, 1215, 1216])
+def test_leaf_indices_of_wide_forests(features):
+    """Up to 1215 used features (32 rows a tile) the device gives the host's leaves for fp32 and half rows; double rows, which the
+    host compares in double, are the device's up to 156 and the host's beyond."""
+    rng = np.random.RandomState(features)
+    X = rng.randn(1000, features).astype(np.float16).astype(np.float32)
+    # two halves of one feature each round: a round per feature, and every feature is used
+    trees = features
+    body = "".join(f"Tree={j}\nnum_leaves=3\nnum_cat=0\nsplit_feature={j} {(j * 7 + 3) % features}\nthreshold={float(np.median(X[:, j]))!r} 0.25\ndecision_type=2 2\n"
+                   f"left_child=1 -1\nright_child=-2 -3\nleaf_value=0.5 -0.25 0.125\nis_linear=0\nshrinkage=1\n\n\n" for j in range(trees))
+    bst = fb.Booster(model_str=f"tree\nversion=v4\nnum_class=1\nnum_tree_per_iteration=1\nlabel_index=0\nmax_feature_idx={features - 1}\nobjective=regression\n"
+                               f"feature_names={' '.join(f'Column_{j}' for j in range(features))}\nfeature_infos={' '.join(['[-5:5]'] * features)}\n\n{body}end of trees\n")
+    host = np.asarray(bst.predict(X, pred_leaf=True)).reshape(len(X), -1)
+    for dtype in (torch.float32, torch.float16, torch.float64):
+        x = torch.from_numpy(X).cuda().to(dtype)
+        rc, leaf = _device_leaves(bst, x, trees)
+        assert (rc == 0) == (features <= (156 if dtype is torch.float64 else 1215))
+        if rc == 0:
+            assert np.array_equal(leaf, host)
+        if dtype is not torch.float16 or rc == 0:   # (half rows on the host are no input of the library)
+            assert np.array_equal(bst.predict(x, pred_leaf=True).cpu().numpy().reshape(len(X), -1), host)
