@@ -93,15 +93,6 @@ std::vector<std::vector<int>> BundleGreedy(const std::vector<int>& order, const 
 template <typename T>
 inline double ReadAs(const void* p, size_t i) { return static_cast<double>(static_cast<const T*>(p)[i]); }
 
-inline double HalfToDouble(uint16_t h) {
-  uint32_t sign = (h >> 15) & 1, exp = (h >> 10) & 0x1F, man = h & 0x3FF;
-  double v;
-  if (exp == 0) v = std::ldexp(static_cast<double>(man), -24);
-  else if (exp == 31) v = man ? std::numeric_limits<double>::quiet_NaN() : std::numeric_limits<double>::infinity();
-  else v = std::ldexp(static_cast<double>(man | 0x400), static_cast<int>(exp) - 25);
-  return sign ? -v : v;
-}
-
 inline double ReadValue(const void* data, int dtype, size_t i) {
   switch (dtype) {
     case kF32: return ReadAs<float>(data, i);

@@ -758,6 +758,7 @@ void GBDT::PredictMat(const void* data, int dtype, int nrow, int ncol, bool row_
           case kU8: row[j] = static_cast<const uint8_t*>(data)[src]; break;
           case kU16: row[j] = static_cast<const uint16_t*>(data)[src]; break;
           case kI32: row[j] = static_cast<const int32_t*>(data)[src]; break;
+          case kF16: row[j] = HalfToDouble(static_cast<const uint16_t*>(data)[src]); break;
           default: row[j] = 0.0;
         }
       }

@@ -135,6 +135,14 @@ class Dataset {
 
 // dtype codes shared with the Python layer
 enum DType : int { kF32 = 0, kF64 = 1, kI8 = 2, kI16 = 3, kU8 = 4, kU16 = 5, kF16 = 6, kI32 = 7 };
+inline double HalfToDouble(uint16_t h) {
+  uint32_t sign = (h >> 15) & 1, exp = (h >> 10) & 0x1F, man = h & 0x3FF;
+  double v;
+  if (exp == 0) v = std::ldexp(static_cast<double>(man), -24);
+  else if (exp == 31) v = man ? std::numeric_limits<double>::quiet_NaN() : std::numeric_limits<double>::infinity();
+  else v = std::ldexp(static_cast<double>(man | 0x400), static_cast<int>(exp) - 25);
+  return sign ? -v : v;
+}
 
 // Text file loader (CSV / TSV / LibSVM with optional header, label/weight/group columns).
 Dataset* LoadDatasetFromFile(const std::string& path, const Config& cfg, const Dataset* reference);

@@ -525,3 +525,20 @@ def test_quantized_training_keeps_monotone_and_interaction_constraints_on_the_ho
         p = {"objective": "regression", "num_leaves": 31, "verbose": -1, "interaction_constraints": [[0, 1], [2, 3]], "quant_mode": quant, "device_type": "cpu"}
         sets = _branch_feature_sets(fb.train(p, fb.Dataset(X, z), 10))
         assert all(s <= {0, 1} or s <= {2, 3} for s in sets), quant
+
+
+@pytest.mark.parametrize("dtype", ["float16", "float64", "int8", "int16", "int32", "uint8", "uint16"])
+def test_host_prediction_reads_every_input_type(dtype):
+    rng = np.random.RandomState(4)
+    X = rng.randint(0, 100, size=(500, 6)).astype(np.float32)
+    y = (X[:, 0] + X[:, 1] > 100).astype(np.float32)
+    bst = fb.train({"objective": "binary", "num_leaves": 15, "verbosity": -1, "device_type": "cpu"}, fb.Dataset(X, y), 5)
+    expected = bst.predict(X)
+    assert len(np.unique(expected)) > 2
+    for order in ("C", "F"):
+        assert np.array_equal(bst.predict(np.asarray(X.astype(dtype), order=order)), expected)
+    if dtype == "float16":
+        # halves on both sides of the thresholds: subnormal, signed, infinite and NaN values as their fp32 twins
+        v = np.array([0.0, -0.0, 6e-8, -6e-8, 1e-4, 65504, np.inf, -np.inf, np.nan, -2.5], dtype=np.float16)
+        Z = rng.choice(v, size=(400, 6)); W = np.where(rng.rand(400, 6) < 0.5, Z, X[:400].astype(np.float16))
+        assert np.array_equal(bst.predict(W), bst.predict(W.astype(np.float32)))
