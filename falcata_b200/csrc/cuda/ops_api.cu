@@ -122,7 +122,8 @@ int FB_OpPartition(const uint8_t* rows, int row_stride, const int* idx, int coun
   DevBuf<int> chunk_left; chunk_left.Alloc(sp.num_chunks + 1); DevBuf<int> left_total; left_total.Alloc(1); DevBuf<HistTask> tasks; tasks.Alloc(1);
   PartArgs a = PartArgs(); a.rows = rows; a.row_stride = row_stride; a.cols = nullptr; a.col_stride = 0; a.idx[0] = const_cast<int*>(idx); a.idx[1] = out_idx; a.splits = d_sp.get(); a.num_splits = 1; a.total_chunks = sp.num_chunks;
   a.bits = bits.get(); a.chunk_left = chunk_left.get(); a.split_left_total = left_total.get(); a.leaves = d_leaves2.get(); a.child_init = d_ci.get(); a.hist_tasks = tasks.get(); a.rows_per_block = 2048;
-  LaunchPartitionFlags(a, s); LaunchPartitionScanSetup(a, s); LaunchPartitionScatter(a, s);
+  FB_CUDA(cudaMemsetAsync(left_total.get(), 0xFF, sizeof(int), s));   // the set-up step writes it, also for no rows
+  LaunchPartition(a, s);
   FB_CUDA(cudaMemcpyAsync(left_count, left_total.get(), sizeof(int), cudaMemcpyDeviceToHost, s));
   FB_CUDA(cudaStreamSynchronize(s));
   OPS_END();

@@ -303,12 +303,13 @@ __global__ void InitIndicesKernel(int* idx, int n) { const int i = blockIdx.x * 
 }  // namespace
 
 void LaunchPartition(const PartArgs& a, cudaStream_t s) {
-  if (a.total_chunks <= 0) return;
   if (a.chunk_words != nullptr) {
+    if (a.total_chunks <= 0) return;   // (the device controller gives every split a chunk)
     LaunchChained(a.world <= 1, PartitionKernel, dim3(a.total_chunks), dim3(kPartThreads), 0, s, a);
     FB_LAUNCHED(); FB_KERNEL_CHECK();
     return;
   }
+  // a split of no rows - a rank of several whose rows are all elsewhere - has no chunk, but its children's records and counts are still due
   LaunchPartitionFlags(a, s); LaunchPartitionScanSetup(a, s); LaunchPartitionScatter(a, s);
 }
 void LaunchPartitionFlags(const PartArgs& a, cudaStream_t s) {

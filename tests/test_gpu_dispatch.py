@@ -102,6 +102,14 @@ def test_one_launch_partition_gives_the_same_model(n, extra):
     assert models[0] == models[1]
 
 
+def test_partition_of_no_rows_sets_up_the_children():
+    """A rank of several may hold none of a split's rows: there is nothing to move, but the left count (zero) is due."""
+    from falcata_b200 import ops
+    rows = torch.zeros(4, 16, dtype=torch.uint8, device="cuda")
+    out, left = ops.partition(rows, torch.empty(0, dtype=torch.int32, device="cuda"), 0, 3)
+    assert out.numel() == 0 and left == 0
+
+
 @pytest.mark.parametrize("flip", ["fused_scan:off", "fused_tail:off,fused_scan:off", "device_controller:off"])
 @pytest.mark.parametrize("max_bin", [15, 63])
 @pytest.mark.parametrize("n", [2049, 30000, 150001])
