@@ -379,7 +379,7 @@ Tree* CudaEngine::TrainTree(int class_id, int tree_index) {
     pa.splits = ca.splits; pa.bits = bits_.get(); pa.chunk_left = chunk_left_.get();
     pa.split_left_total = split_left_total_.get(); pa.leaves = leaves_.get(); pa.child_init = ca.child_init; pa.hist_tasks = hist_tasks_.get(); pa.rows_per_block = rpb;
     pa.world = dp ? world_ : 1;
-    pa.chunk_words = one_launch_part ? chunk_words_.get() : nullptr; pa.rights_down = 1;
+    pa.chunk_words = one_launch_part ? chunk_words_.get() : nullptr; pa.look_back_polls = kLookbackPolls; pa.rights_down = 1;
     if (dp) for (int r = 0; r < world_; ++r) pa.peer_counts[r] = fabric_->Ptr<int>(r, off_counts_) + static_cast<size_t>(rank_) * NL;
     if (feature_parallel_) SetupBitmapBroadcast(&pa);
     ha.identity_root = 0; ha.rows_per_block = rpb;

@@ -235,6 +235,7 @@ void LaunchGatherBest(const FindArgs& a, cudaStream_t s);      // world > 1: arg
 
 // ------------------------------------------------------------- partition ----
 constexpr int kPartChunk = 2048;
+constexpr int kLookbackPolls = 1 << 12;   // of a predecessor's word; then its count is taken from its rows: no wait depends on another block
 struct alignas(16) ChildInit {     // host-decided child bookkeeping of one split
   int left_slot, right_slot;       // histogram slots of the children
   int smaller_is_left;
@@ -259,6 +260,7 @@ struct PartArgs {
   int world; int* peer_counts[kMaxRanks];   // world > 1: address of counts[this rank][0] inside every rank's heap
   const LevelCtrl* ctrl;     // non-null: num_splits / total_chunks come from the device controller
   unsigned long long* chunk_words;   // non-null: one launch per level; [chunks] look-back words, valid when they carry `epoch`
+  int look_back_polls;               // one-launch form: kLookbackPolls (0: a chunk counts its predecessors' rows itself at once)
   unsigned int epoch;                // one-launch form: differs from that of every earlier launch on the same words (never 0)
   int rights_down;                   // three-launch form: rights from the window's end downwards, the order of the one-launch form (0: stable)
   int identity;                      // one-launch form: the windows hold the rows in order (root of an unbagged tree), idx is not read

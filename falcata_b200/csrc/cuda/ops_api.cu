@@ -17,6 +17,32 @@ std::vector<HistPartition> MakePartitions(const std::vector<int>& gstart, const 
   }
   return parts;
 }
+// polls < 0: the three-launch form
+void PartitionOp(const uint8_t* rows, int row_stride, const int* idx, int count, int group, int threshold, int default_left, int missing_type, int default_bin, int num_bin,
+                 int polls, int* out_idx, int* left_count) {
+  cudaStream_t s = 0;
+  PartSplit sp; memset(&sp, 0, sizeof(sp));
+  sp.leaf = 0; sp.right_leaf = 1; sp.begin = 0; sp.count = count; sp.buffer = 0; sp.group = group; sp.num_bin = num_bin; sp.threshold = threshold; sp.default_left = default_left;
+  sp.missing_type = missing_type; sp.default_bin = default_bin; sp.chunk_begin = 0; sp.num_chunks = (count + kPartChunk - 1) / kPartChunk;
+  ChildInit ci; memset(&ci, 0, sizeof(ci)); ci.left_slot = 0; ci.right_slot = 1; ci.smaller_is_left = 1; ci.hist_num_blocks = 1;
+  LeafInfo leaf; memset(&leaf, 0, sizeof(leaf)); leaf.count = count;
+  DevBuf<PartSplit> d_sp; d_sp.Upload(&sp, 1, s); DevBuf<ChildInit> d_ci; d_ci.Upload(&ci, 1, s);
+  DevBuf<LeafInfo> d_leaves; d_leaves.Alloc(2); d_leaves.Upload(&leaf, 1, s); d_leaves.Alloc(2);
+  DevBuf<LeafInfo> d_leaves2; d_leaves2.Alloc(2); FB_CUDA(cudaMemcpyAsync(d_leaves2.get(), d_leaves.get(), sizeof(LeafInfo), cudaMemcpyDeviceToDevice, s));
+  DevBuf<unsigned int> bits; bits.Alloc(static_cast<size_t>(sp.num_chunks + 1) * (kPartChunk / 32));
+  DevBuf<int> chunk_left; chunk_left.Alloc(sp.num_chunks + 1); DevBuf<int> left_total; left_total.Alloc(1); DevBuf<HistTask> tasks; tasks.Alloc(1);
+  PartArgs a = PartArgs(); a.rows = rows; a.row_stride = row_stride; a.cols = nullptr; a.col_stride = 0; a.idx[0] = const_cast<int*>(idx); a.idx[1] = out_idx; a.splits = d_sp.get(); a.num_splits = 1; a.total_chunks = sp.num_chunks;
+  a.bits = bits.get(); a.chunk_left = chunk_left.get(); a.split_left_total = left_total.get(); a.leaves = d_leaves2.get(); a.child_init = d_ci.get(); a.hist_tasks = tasks.get(); a.rows_per_block = 2048;
+  FB_CUDA(cudaMemsetAsync(left_total.get(), 0xFF, sizeof(int), s));   // the set-up step writes it, also for no rows
+  DevBuf<unsigned long long> words;
+  if (polls >= 0) {
+    words.Alloc(sp.num_chunks); words.Zero(s);
+    a.chunk_words = words.get(); a.epoch = 1; a.look_back_polls = polls; a.identity = idx == nullptr ? 1 : 0; a.world = 1;
+  }
+  LaunchPartition(a, s);
+  FB_CUDA(cudaMemcpyAsync(left_count, left_total.get(), sizeof(int), cudaMemcpyDeviceToHost, s));
+  FB_CUDA(cudaStreamSynchronize(s));
+}
 }  // namespace
 
 #define OPS_BEGIN() try {
@@ -105,27 +131,21 @@ int FB_OpQuantize(const float* grad, const float* hess, int n, int bins, int sto
   OPS_END();
 }
 
-// Stable partition of idx[0..count) by "bin(row, group) <= threshold"; writes the result to out_idx and the left count to *left_count (host).
+// Partition of idx[0..count) by "bin(row, group) <= threshold"; writes the result to out_idx and the left count to *left_count (host).
+// FB_OpPartition: the three-launch form, stable in both children.
 int FB_OpPartition(const uint8_t* rows, int row_stride, const int* idx, int count, int group, int threshold, int default_left, int missing_type, int default_bin,
                    int num_bin, int* out_idx, int* left_count) {
   OPS_BEGIN();
-  cudaStream_t s = 0;
-  PartSplit sp; memset(&sp, 0, sizeof(sp));
-  sp.leaf = 0; sp.right_leaf = 1; sp.begin = 0; sp.count = count; sp.buffer = 0; sp.group = group; sp.num_bin = num_bin; sp.threshold = threshold; sp.default_left = default_left;
-  sp.missing_type = missing_type; sp.default_bin = default_bin; sp.chunk_begin = 0; sp.num_chunks = (count + kPartChunk - 1) / kPartChunk;
-  ChildInit ci; memset(&ci, 0, sizeof(ci)); ci.left_slot = 0; ci.right_slot = 1; ci.smaller_is_left = 1; ci.hist_num_blocks = 1;
-  LeafInfo leaf; memset(&leaf, 0, sizeof(leaf)); leaf.count = count;
-  DevBuf<PartSplit> d_sp; d_sp.Upload(&sp, 1, s); DevBuf<ChildInit> d_ci; d_ci.Upload(&ci, 1, s);
-  DevBuf<LeafInfo> d_leaves; d_leaves.Alloc(2); d_leaves.Upload(&leaf, 1, s); d_leaves.Alloc(2);
-  DevBuf<LeafInfo> d_leaves2; d_leaves2.Alloc(2); FB_CUDA(cudaMemcpyAsync(d_leaves2.get(), d_leaves.get(), sizeof(LeafInfo), cudaMemcpyDeviceToDevice, s));
-  DevBuf<unsigned int> bits; bits.Alloc(static_cast<size_t>(sp.num_chunks + 1) * (kPartChunk / 32));
-  DevBuf<int> chunk_left; chunk_left.Alloc(sp.num_chunks + 1); DevBuf<int> left_total; left_total.Alloc(1); DevBuf<HistTask> tasks; tasks.Alloc(1);
-  PartArgs a = PartArgs(); a.rows = rows; a.row_stride = row_stride; a.cols = nullptr; a.col_stride = 0; a.idx[0] = const_cast<int*>(idx); a.idx[1] = out_idx; a.splits = d_sp.get(); a.num_splits = 1; a.total_chunks = sp.num_chunks;
-  a.bits = bits.get(); a.chunk_left = chunk_left.get(); a.split_left_total = left_total.get(); a.leaves = d_leaves2.get(); a.child_init = d_ci.get(); a.hist_tasks = tasks.get(); a.rows_per_block = 2048;
-  FB_CUDA(cudaMemsetAsync(left_total.get(), 0xFF, sizeof(int), s));   // the set-up step writes it, also for no rows
-  LaunchPartition(a, s);
-  FB_CUDA(cudaMemcpyAsync(left_count, left_total.get(), sizeof(int), cudaMemcpyDeviceToHost, s));
-  FB_CUDA(cudaStreamSynchronize(s));
+  PartitionOp(rows, row_stride, idx, count, group, threshold, default_left, missing_type, default_bin, num_bin, -1, out_idx, left_count);
+  OPS_END();
+}
+// The one-launch form: lefts in order, rights in reverse order. idx null: rows 0..count-1. polls: how often a chunk asks for a
+// predecessor's count before it counts that chunk's rows itself.
+int FB_OpPartitionOneLaunch(const uint8_t* rows, int row_stride, const int* idx, int count, int group, int threshold, int default_left, int missing_type,
+                            int default_bin, int num_bin, int polls, int* out_idx, int* left_count) {
+  OPS_BEGIN();
+  if (polls < 0 || count <= 0) Log::Fatal("FB_OpPartitionOneLaunch: polls must not be negative and there must be rows (got %d, %d)", polls, count);
+  PartitionOp(rows, row_stride, idx, count, group, threshold, default_left, missing_type, default_bin, num_bin, polls, out_idx, left_count);
   OPS_END();
 }
 

@@ -159,16 +159,15 @@ __device__ __forceinline__ unsigned long long ChunkWord(unsigned int epoch, bool
 __device__ __forceinline__ void StoreChunkWord(unsigned long long* p, unsigned long long w) { asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(w) : "memory"); }
 __device__ __forceinline__ unsigned long long LoadChunkWord(const unsigned long long* p) { unsigned long long w; asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(w) : "l"(p) : "memory"); return w; }
 
-constexpr int kLookbackPolls = 1 << 12;   // then the count is taken from the rows themselves: no wait depends on another block
-
 // Lefts before local chunk `chunk` of a split; one warp, all lanes. words: the split's first chunk word.
 __device__ int LookBack(const PartArgs& a, const PartSplit& sp, const unsigned long long* words, int chunk) {
   const int lane = threadIdx.x & 31;
   int before = 0;
   for (int c = chunk - 1; c >= 0; c -= 32) {
     const int mine = c - lane;   // lane 0: the nearest predecessor
-    unsigned long long w = 0; bool ready = mine < 0; unsigned int inclusive = 0, missing = 0;
-    for (int poll = 0; poll < kLookbackPolls; ++poll) {
+    unsigned long long w = 0; bool ready = mine < 0; unsigned int inclusive = 0;
+    unsigned int missing = a.look_back_polls > 0 ? 0u : __ballot_sync(0xffffffffu, !ready);
+    for (int poll = 0; poll < a.look_back_polls; ++poll) {
       if (!ready) { w = LoadChunkWord(words + mine); ready = static_cast<unsigned int>(w >> 32) == a.epoch; }
       inclusive = __ballot_sync(0xffffffffu, ready && mine >= 0 && (w & 0x80000000ull) != 0);
       missing = __ballot_sync(0xffffffffu, !ready);

@@ -58,6 +58,16 @@ def partition(rows: torch.Tensor, idx: torch.Tensor, group: int, threshold: int,
     return out, left.value
 
 
+def partition_one_launch(rows: torch.Tensor, idx: Optional[torch.Tensor], group: int, threshold: int, default_left: bool = True, missing_type: int = 0,
+                         default_bin: int = 0, num_bin: int = 256, polls: int = 4096) -> Tuple[torch.Tensor, int]:
+    """The training path's one-launch partition: lefts in order from the start, rights from the end. ``idx`` None: all rows in order."""
+    count = rows.shape[0] if idx is None else idx.numel()
+    out = torch.empty(count, dtype=torch.int32, device=rows.device)
+    left = ctypes.c_int(0)
+    _check(_lib().FB_OpPartitionOneLaunch(_p(rows), rows.shape[1], _p(idx), count, group, threshold, 1 if default_left else 0, missing_type, default_bin, num_bin, int(polls), _p(out), ctypes.byref(left)))
+    return out, left.value
+
+
 def launch_count() -> int:
     out = ctypes.c_longlong(0)
     _lib().FB_OpLaunchCount(ctypes.byref(out))

@@ -102,6 +102,23 @@ def test_one_launch_partition_gives_the_same_model(n, extra):
     assert models[0] == models[1]
 
 
+@pytest.mark.parametrize("polls", [0, 1, 4096])
+@pytest.mark.parametrize("n", [1, 2047, 2048, 2049, 32 * 2048, 33 * 2048 + 1, 65 * 2048 + 5, 400001])
+def test_one_launch_partition(n, polls):
+    """Windows of one chunk, of a whole look-back window (32 chunks before the last) and of several. Without polls every chunk
+    counts the rows of all chunks before it: the way out of a wait for a predecessor that does not publish."""
+    from falcata_b200 import ops
+    gen = torch.Generator(device="cuda"); gen.manual_seed(n)
+    rows = torch.randint(0, 64, (n, 16), generator=gen, device="cuda", dtype=torch.int32).to(torch.uint8)
+    perm = torch.randperm(n, generator=gen, device="cuda").int()
+    for idx in (None, perm):
+        order = torch.arange(n, device="cuda", dtype=torch.int32) if idx is None else idx
+        for threshold in (-1, 20, 63):
+            out, left = ops.partition_one_launch(rows, idx, 5, threshold, num_bin=64, polls=polls)
+            go_left = rows[order.long(), 5].int() <= threshold
+            assert left == int(go_left.sum()) and torch.equal(out, torch.cat([order[go_left], order[~go_left].flip(0)]))
+
+
 def test_partition_of_no_rows_sets_up_the_children():
     """A rank of several may hold none of a split's rows: there is nothing to move, but the left count (zero) is due."""
     from falcata_b200 import ops
