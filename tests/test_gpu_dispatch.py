@@ -174,6 +174,29 @@ def test_split_search_agrees_with_the_host(features, max_bin):
     assert device == trained(device_type="cpu")
 
 
+@pytest.mark.parametrize("missing", ["none", "nan", "zero"])
+@pytest.mark.parametrize("features", [1, 9, 17])
+@pytest.mark.parametrize("max_bin", [7, 32, 33, 64, 65, 128, 129, 255])
+def test_fp32_split_search_agrees_with_the_host(max_bin, features, missing):
+    """fp64 prefix sums over staged fp32 histograms: runs of 1 to 8 bins per lane, with the bin of missing values at the end
+    (NaN) or inside (zero). The gradients lie on a coarse grid, so all sums are exact and both learners see the same ones."""
+    rng = np.random.RandomState(features * 1000 + max_bin)
+    X = rng.randn(3000, features).astype(np.float32)
+    if missing != "none":
+        X[rng.rand(*X.shape) < 0.1] = np.nan if missing == "nan" else 0.0
+    y = (np.round((np.nan_to_num(X).sum(axis=1) + np.isnan(X[:, 0]) + rng.randn(3000)) * 8) / 8).astype(np.float32)
+    p = {"objective": "none", "num_leaves": 31, "max_bin": max_bin, "verbosity": -1, "quant_mode": "none", "min_data_in_leaf": 5, "grow_policy": "level"}
+
+    def trained(**kw):
+        bst = fb.Booster(dict(p, **kw), fb.Dataset(X, y, params={"max_bin": max_bin, "zero_as_missing": missing == "zero"}))
+        bst.update(fobj=lambda preds, ds: (-y, np.ones_like(y)))
+        return model_body(bst.model_to_string())
+
+    device = trained(device_type="cuda")
+    assert device == trained(device_type="cuda", cuda_plan="auto,fused_tail:off")
+    assert device == trained(device_type="cpu")
+
+
 @pytest.mark.parametrize("zero_as_missing", [False, True])
 @pytest.mark.parametrize("quant", ["fixedpoint", "none"])
 @pytest.mark.parametrize("levels", [20, 33, 66, 130, 200])
@@ -297,3 +320,33 @@ def test_leaf_indices_of_wide_forests(features):
         if rc == 0:
             assert np.array_equal(leaf, host)
         assert np.array_equal(bst.predict(x, pred_leaf=True).cpu().numpy().reshape(len(X), -1), host)
+
+
+@pytest.mark.parametrize("norm", [True, False])
+@pytest.mark.parametrize("sizes,levels", [([1, 2, 29, 30, 31, 33, 64], 5), ([128, 1, 90], 5), ([600, 3], 5), ([40, 65], 70)])
+@pytest.mark.parametrize("truncation", [1, 30, 31, 64, 1000])
+def test_lambdarank_pairs_agree_with_the_host(truncation, sizes, levels, norm, monkeypatch):
+    """Gradients of single documents at truncations below, at and above the query lengths: the tree puts every document into a
+    leaf of its own, so the new scores are -g / (h + 1) of that document. (600 documents: blocks of 256 threads; 70 label levels:
+    the scan instead of the counts.)"""
+    rng = np.random.RandomState(truncation + len(sizes))
+    n = sum(sizes)
+    X = np.column_stack([np.arange(n) // 25, np.arange(n) % 25]).astype(np.float32)
+    y = rng.randint(0, levels, size=n).astype(np.float32)
+    start = rng.randn(n)
+    p = {"objective": "lambdarank", "num_leaves": 1000, "max_bin": 255, "min_data_in_leaf": 1, "min_sum_hessian_in_leaf": 0, "lambda_l2": 1.0, "learning_rate": 1.0, "verbosity": -1,
+         "quant_mode": "none", "device_type": "cuda", "grow_policy": "level", "lambdarank_truncation_level": truncation, "lambdarank_norm": norm, "boost_from_average": False,
+         "label_gain": ",".join(str(2 ** k - 1 if levels <= 31 else k) for k in range(levels))}
+
+    def scores():
+        data = fb.Dataset(X, y, group=np.asarray(sizes, dtype=np.int32), init_score=start, params={"min_data_in_bin": 1, "max_bin": 255})
+        bst = fb.train(p, data, 1, keep_training_booster=True)
+        return bst.train_score_tensor().cpu().numpy().reshape(-1) - start.astype(np.float32)
+
+    device = scores()
+    monkeypatch.setenv("FALCATA_HOST_GRADIENTS", "1")
+    host = scores()
+    assert np.count_nonzero(host) > 0
+    # a document's sums run over up to 600 fp32 pairs on the device, and the step is the difference of two fp32 scores of up to 10:
+    # 600 x 2^-24 of the step and 2^-20. A truncation off by one moves a hundred documents or more, most by 1e-3 and up
+    np.testing.assert_allclose(device, host, rtol=1e-4, atol=1e-5)
