@@ -360,8 +360,8 @@ void CudaEngine::SetupOwnership() {
   h_bin_owner_ = owner;
 }
 
-// Gradient levels actually used. The global histograms keep 32-bit halves per bin, so rows x levels must stay below
-// 2^31 over ALL ranks' rows; a default count that breaks this is lowered, an explicit one is refused. A default
+// Gradient levels actually used. The global histograms keep 32-bit halves per bin, and the split search adds such words up to
+// the whole leaf's sum (FindSplitsWarp), so rows x levels must stay below 2^31 over ALL ranks' rows; a default count that breaks this is lowered, an explicit one is refused. A default
 // stochastic count (4) is raised where leaves get small on large data, where 4 levels fit rounding noise: to 64 with a
 // constant hessian, else 16; not for multiclass and not for binary labels beyond 50:1, where rare large gradients pin the
 // scale. Every rank takes the same decision (global row count, label counts summed over the ranks).
@@ -405,8 +405,9 @@ void CudaEngine::ResolveQuantBins() {
 int CudaEngine::ChooseRowsPerBlock(long long total_rows) const {
   if (lane_mode_ != 0) {
     // the lane kernel runs one block per SM with a fixed cost per block (tile clear, pipeline fill, merge of
-    // the warps' tiles): aim at about four waves (measured best at 11M and 1.4M rows), in units of 384 rows,
-    // within what the 16-bit lanes of the packed cells allow per warp tile
+    // the warps' tiles): aim at about four waves (measured best at 11M and 1.4M rows), in units of one stage of the block's
+    // warps (32 rows each: 1024 rows in the reduction form, 320 to 640 otherwise), within what the 16-bit lanes of the
+    // packed cells allow per warp tile
     const int unit = LaneRowsUnit(lane_red_, sub_rows_, lane_bins_, !quant_);   // rows of one stage across the block's warps
     long long rpb = (total_rows / (4LL * num_sms_) + unit - 1) / unit * unit;
     if (!quant_) {

@@ -124,7 +124,7 @@ class CudaEngine : public DeviceEngine {
   DevBuf<char> level_blob_; PinnedBuf<char> h_level_blob_;
   DevBuf<HistTask> hist_tasks_; DevBuf<unsigned int> hist_status_; PinnedBuf<unsigned int> h_hist_status_;
   DevBuf<unsigned int> bits_; DevBuf<int> chunk_left_, split_left_total_;
-  DevBuf<unsigned long long> chunk_words_; unsigned int part_epoch_ = 0;   // look-back words of the one-launch partition, epoch of its last launch
+  DevBuf<unsigned long long> chunk_words_; unsigned int part_epoch_ = 0;   // look-back words of the one-launch partition, epoch of its last launch (32 bits: 10^8 trees and more)
   DevBuf<int> features_, sub_features_;
   // exact leaf-wise growth (grow_policy=leaf): the device grows up to grow_leaves_ leaves, the host keeps the best num_leaves
   bool leafwise_ = false; int grow_leaves_ = 0;

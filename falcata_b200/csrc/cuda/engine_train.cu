@@ -1,11 +1,13 @@
 // Device engine: one boosting iteration and the level loop of one tree.
 //
-// Per level (all splitting leaves at once): partition flags -> scan + child/leaf/task setup ->
-// scatter -> construct (smaller children; the epilogue adds each bin into the slot of the rank that
-// owns its feature) -> find on the owned slice (+ in-place larger = parent - smaller) -> per-leaf
-// argmax (multi-rank: stored into every peer, then an argmax over the ranks' records) -> ONE
-// read-back of the leaf records and best splits, on which the host applies the gain-ranked leaf
-// budget. Exact child counts come back with that read-back: no second synchronisation per level.
+// Per level (all splitting leaves at once): partition with the children's set-up (one launch; feature-parallel, the host-driven
+// loop and fused_scan:off: flags -> scan + set-up -> scatter) -> construct (smaller children; the epilogue adds each bin into the
+// slot of the rank that owns its feature) -> search on the owned slice (+ in-place larger = parent - smaller), whose last block
+// takes the per-leaf argmax (multi-rank: stored into every peer, then an argmax over the ranks' records) and runs the level
+// controller: gain-ranked leaf budget, the next level's splits. The host enqueues a tree's levels ahead and reads the journal
+// and the leaf records back once per tree.
+// Host-driven loop (device_controller:off, forced splits, more than 1024 leaves): one read-back of the leaf records and best
+// splits per level, on which the host applies the budget; exact child counts come back with it.
 //
 // Multi-rank ordering (all inside kernels, no NCCL): construct's last block raises "construct done"
 // on every peer; the split search waits for all ranks' flags; its last block raises "best published";
