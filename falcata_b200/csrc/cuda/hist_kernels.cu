@@ -88,7 +88,8 @@ __device__ inline bool PushTaskIfLast(const HistArgs& a, int ti, const HistTask&
 // ranks), kBins bins of up to 32 groups at a time. The tiles hold a bin's groups side by side, the histogram a group's bins: a
 // transpose in shared memory (`stage`, free by now: kBytes) makes the global adds run along the bins. Added cell by
 // cell from the tiles' order they are 32 different sectors per instruction, 16k of them per block of 255-bin fp32 sums.
-// Measured (mean launch of a tree): 1M x 100 groups of 255 bins, fp32, 156 -> 116 us; 515k x 90, integer, 65 -> 43 us.
+// Measured (mean launch of a tree, with shorter fp32 blocks and the groups' places in shared memory): 1M x 100 groups of 255 bins, fp32,
+// 152 -> 109 us; 515k x 90, integer, 71 -> 35 us; 10k x 28, fp32, 30 -> 16 us.
 // A task with a single block stores (its cells were cleared with the pool; nobody else adds to them). All threads of the block
 // call Write between two rounds of Put.
 // (start, count): the groups' places in the bin space, in shared memory since the block's start - the tiles leave the SM a few
@@ -551,7 +552,7 @@ __global__ void __launch_bounds__(kHistThreads) HistFloatKernel(HistArgs a) {
 // Compact view: kGatherRows rows x 32 output bytes (32 listed groups, or 64 when two share a byte) per block. The columns come
 // in as 16-byte pieces (16 rows of a group; the column stride is a multiple of 16), are turned in shared memory four rows by
 // four bytes at a time, and leave as whole 32-byte sectors.
-// Bound by memory: bytes in + out. Measured at 1M rows x 200 of 2000 groups, two per byte (200 MB in, 112 MB out): 440 us with
+// Bound by memory: bytes in + out. Measured at 1M rows x 200 of 2000 groups, two per byte (200 MB in, 112 MB out): 445 us with
 // byte loads (a 32-byte sector per warp and load), 135 us.
 constexpr int kGatherRows = 256;
 template <bool PACK4>

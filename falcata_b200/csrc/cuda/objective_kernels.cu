@@ -39,7 +39,7 @@ __device__ inline float SignF(float x) { return (x > 0.f) - (x < 0.f); }
 // Per-row kernels of the round's set-up (gradients, quantization, interleaving) walk the rows with a bounded grid, four
 // rows per thread and step where the buffers allow 16-byte accesses. What bounded the one-row-per-thread form at 11M rows
 // was not the 16 bytes per row but the block ends: 43k blocks x 2 atomics on the same two words, one after the other in L2.
-// A grid of at most kRowBlocks blocks leaves 2.4k of them: gradients 107 -> 36 us, quantization 97 -> 42 us (11M rows).
+// A grid of at most kRowBlocks blocks leaves 2.4k of them: gradients 91 -> 39 us, quantization 97 -> 43 us (11M rows).
 constexpr int kRowThreads = 256;
 constexpr int kRowBlocks = 148 * 8;      // resident at once on 148 SMs
 inline int RowBlocks(int n, int vec) { return std::max(1, std::min(kRowBlocks, (n + kRowThreads * vec - 1) / (kRowThreads * vec))); }
@@ -296,7 +296,7 @@ __global__ void LambdarankKernel(const float* __restrict__ score, const float* _
     __syncthreads();
     // ideal DCG at the truncation level: the gains in descending label order, added position by position in double. The
     // terms (a double logarithm and a division each) come from 32 lanes at once; one thread took 30 of them in a row, during
-    // which the rest of the block waited. (2M documents, queries of 1 to 200: 924 -> 447 us with the shorter pair loop below.)
+    // which the rest of the block waited. (2M documents, queries of 1 to 200: 933 -> 453 us with the shorter pair loop below.)
     if (few_levels) {
       if (threadIdx.x < 32) {
         const int lane = threadIdx.x, npos = min(trunc, cnt);

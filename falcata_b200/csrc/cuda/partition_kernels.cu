@@ -190,8 +190,8 @@ __device__ int LookBack(const PartArgs& a, const PartSplit& sp, const unsigned l
 }
 
 // Bound by the latency of the dependent (row id -> bin byte) load pair: eight row ids, then eight bins are in flight per
-// thread, and 32 registers keep eight blocks on an SM. Measured (mean level, against flags + scan + scatter): 11M rows 94 -> 72 us,
-// 10k rows 17 -> 8 us.
+// thread, and 32 registers keep eight blocks on an SM. Measured (mean level, against flags + scan + scatter): 11M rows 94 -> 75 us,
+// 10k rows 13 -> 8 us.
 __global__ void __launch_bounds__(kPartThreads, 8) PartitionKernel(PartArgs a) {
   ChainWait();
   const int chunk = blockIdx.x;

@@ -7,8 +7,8 @@
 // What bounds it: instructions per step of a walk. A node holds everything as ready-made offsets into the block's shared
 // memory (feature row, left child) and a leaf is a node that leads to itself - its feature row holds -infinity, which goes
 // left everywhere - so a step is shift, mask, load, mask, compare, add, load, without a test for the end.
-// Measured: 4M rows x 136 features, 500 trees of 255 leaves, 41.0 -> 24.4 ms against 256 threads with eight walks each and
-// nodes of indices; 200k rows x 100 features, 500 trees of 127 leaves with missing values, 3.8 -> 2.1 ms.
+// Measured: 4M rows x 136 features, 500 trees of 255 leaves, 41.0 -> 24.6 ms against 256 threads with eight walks each and
+// nodes of indices; 200k rows x 100 features, 500 trees of 127 leaves with missing values, 3.9 -> 2.1 ms.
 //
 // Parity: python-package/falcata/basic.py:L5112-5163 (device predict route: raw score, converted score, leaf index),
 // include/Falcata/tree.h:L361-439 (numerical decision with missing-value handling). Forests with categorical splits, a tree of

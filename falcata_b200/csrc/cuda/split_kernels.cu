@@ -185,8 +185,8 @@ __device__ void ScanCategoricalWarp(const FindArgs& a, const BinSrc& src, char* 
 // flight at once and are staged in shared memory; a lane then owns a run of 1, 2, 4 or 8 consecutive bins, so the warp makes
 // ONE prefix scan over the lane totals instead of one per 32 bins. Integer sums are added as packed 64-bit words, 32 bits a
 // half: no sum of a leaf's rows leaves its half because rows x levels stay below 2^31 (CudaEngine::ResolveQuantBins).
-// Measured with the one-stage tail (mean launch): 10k rows x 28 features of 255 bins 33 -> 20 us, leaf-wise at 1.4M rows 43 -> 26,
-// 200 of 2000 features 157 -> 40 (there mostly for no longer subtracting the features outside the sample).
+// Measured with the one-stage tail (mean launch): 10k rows x 28 features of 255 bins 22 -> 20 us, leaf-wise at 1.4M rows 36 -> 28,
+// 200 of 2000 features 150 -> 40 (there mostly for no longer subtracting the features outside the sample).
 template <bool QUANT>
 __device__ void FindSplitsWarp(const FindArgs& a, int fi, CandLite* out) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
